@@ -34,14 +34,6 @@ struct alignas(32) Box32 {
   int4 idp;    // id, 0, 0, 0
 };
 
-constexpr int kSortThreads = 512;
-constexpr int kSortIpt = kSortTile / kSortThreads;  // 16 keys per thread
-constexpr int kSortWarps = kSortThreads / 32;
-using BuildCtrl = SortCtrl;
-
-constexpr uint64_t kFlagAgg = 1ull << 62;
-constexpr uint64_t kFlagIncl = 2ull << 62;
-
 // ---------------------------------------------------------------------------
 // 1. encode
 // ---------------------------------------------------------------------------
@@ -59,7 +51,6 @@ constexpr int kEncThreads = 256;
 constexpr int kEncGroups = 4;                            // float4 groups per thread
 constexpr int kEncTile = 4 * kEncGroups * kEncThreads;   // 4096 boxes
 constexpr int kGroups = 256;                             // record runs: by the key's top byte
-static_assert(kDigits * kDigitBits - kDigitBits >= 24, "the last digit lies in the top byte");
 static_assert(kGroups <= kEncThreads, "one thread per run");
 
 struct BoxIn {
@@ -104,10 +95,10 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(BoxIn in, int64_t n
                                                              uint32_t* __restrict__ keys,
                                                              uint32_t* __restrict__ slots,
                                                              Box32* __restrict__ aos,
-                                                             uint32_t* __restrict__ hist)
+                                                             SortCtrl* __restrict__ ctrl)
 {
-  // digit histograms over all of this CTA's tiles (the last digit lies in
-  // the top byte: it is added from the tile's top-byte counts)
+  // digit histograms over all of this CTA's tiles (the last digit is the top
+  // byte: it is added from the tile's top-byte counts)
   __shared__ uint32_t sh[kDigits][kBins];
   __shared__ uint32_t s_run[kGroups];  // this tile: count, then run start, per top byte
   __shared__ uint32_t s_wsum[kGroups / 32];
@@ -153,7 +144,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(BoxIn in, int64_t n
     uint32_t cnt = 0, x = 0;
     if (tid < kGroups) {
       cnt = s_run[tid];
-      if (cnt) atomicAdd(&sh[kDigits - 1][key_digit((uint32_t)tid << 24, kDigits - 1)], cnt);
+      if (cnt) atomicAdd(&sh[kDigits - 1][tid], cnt);
       x = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
@@ -205,304 +196,9 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(BoxIn in, int64_t n
   }
   for (int i = tid; i < kDigits * kBins; i += kEncThreads) {
     const uint32_t v = (&sh[0][0])[i];
-    if (v) atomicAdd(&hist[i], v);
+    if (v) atomicAdd(&ctrl->hist[i], v);
   }
-}
-
-// ---------------------------------------------------------------------------
-// 2. plan
-// ---------------------------------------------------------------------------
-// One warp per digit: a digit whose histogram has one bin holding every key
-// is uniform and its pass is skipped (a stable pass over a uniform digit
-// leaves the order unchanged); the exclusive prefix of the bins is each
-// bucket's global start.
-__global__ void plan_kernel(const uint32_t* __restrict__ hist, int64_t n, BuildCtrl* ctrl)
-{
-  __shared__ int s_uniform[kDigits];
-  if (threadIdx.x < kDigits) s_uniform[threadIdx.x] = 0;
-  __syncthreads();
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (w < kDigits) {
-    const int nb = 1 << digit_bits(w);
-    uint32_t carry = 0;
-    for (int c = 0; c < nb; c += 32) {
-      const bool in = c + l < nb;
-      const uint32_t v = in ? hist[w * kBins + c + l] : 0u;
-      if (in && (int64_t)v == n) s_uniform[w] = 1;
-      uint32_t x = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (l >= o) x += y;
-      }
-      if (in) ctrl->bucket_start[w * kBins + c + l] = (int)(carry + x - v);
-      carry += __shfl_sync(0xffffffffu, x, 31);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int act = 0, na = 0;
-    for (int d = 0; d < kDigits; d++)
-      if (!s_uniform[d]) { act |= 1 << d; na++; }
-    ctrl->active = act;
-    ctrl->n_active = na;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// 3. onesweep pass
-// ---------------------------------------------------------------------------
-// Lanes of the warp whose value equals this lane's (v < 2^kBits), from one
-// ballot per bit; on this part it issues faster than __match_any_sync
-// (measured over the four 8-bit passes of a 100M-key build: 3.7 ms against
-// 4.3 ms).
-template <int kBits>
-__device__ __forceinline__ uint32_t peer_mask(uint32_t v)
-{
-  uint32_t peers = 0xffffffffu;
-#pragma unroll
-  for (int b = 0; b < kBits; b++) {
-    const bool bit = (v >> b) & 1u;
-    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-    peers &= bit ? bal : ~bal;
-  }
-  return peers;
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p)
-{
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// Shared memory of one pass over a kBits-bit digit: keys and values staged in
-// destination order, the tile's incoming values prefetched while the tile is
-// ranked (narrow digits only: with 1024 bins the per-warp counters take that
-// room, and the values are copied straight to their staged slots instead),
-// the per-warp digit counters (16-bit: at most 8192 per tile), the bins'
-// global offsets and the warp sums of the bin scan.
-template <int kBits>
-struct SweepSmem {
-  static constexpr int kB = 1 << kBits;
-  static constexpr bool kPrefetch = kBits <= 8;
-  static constexpr size_t kKeys = 0;
-  static constexpr size_t kVals = kKeys + 4 * (size_t)kSortTile;
-  static constexpr size_t kVin = kVals + 4 * (size_t)kSortTile;
-  static constexpr size_t kHist = kVin + (kPrefetch ? 4 * (size_t)kSortTile : 0);
-  static constexpr size_t kGbase = kHist + 2 * (size_t)kSortWarps * (kB < 2 ? 2 : kB);
-  static constexpr size_t kWsum = kGbase + 4 * (size_t)kB;
-  static constexpr size_t kBytes = kWsum + 4 * 32;
-};
-static_assert(2 * (SweepSmem<10>::kBytes + 1024) <= 227 * 1024, "two 10-bit CTAs per SM");
-static_assert(2 * (SweepSmem<8>::kBytes + 1024) <= 227 * 1024, "two 8-bit CTAs per SM");
-
-// Ranks this thread's keys inside its warp, stably (rounds in order, lanes in
-// order).  kFull: every item of the tile is valid (no bounds checks, and the
-// digit fits kBits bits); otherwise invalid items take digit 2^kBits.
-template <bool kFull, int kBits>
-__device__ __forceinline__ void rank_keys(const uint32_t (&key)[kSortIpt], uint32_t (&rank)[kSortIpt],
-                                          uint16_t* wh, int wbase, int tile_n, int shift)
-{
-  constexpr uint32_t kMask = (1u << kBits) - 1u;
-  const uint32_t lt = lanemask_lt();
-#pragma unroll
-  for (int i = 0; i < kSortIpt; i++) {
-    const bool v = kFull || wbase + 32 * i < tile_n;
-    const uint32_t dig = v ? (key[i] >> shift) & kMask : kMask + 1u;
-    const uint32_t peers = kFull ? peer_mask<kBits>(dig) : peer_mask<kBits + 1>(dig);
-    const uint32_t old = v ? wh[dig] : 0u;
-    __syncwarp();
-    if (v && (peers & lt) == 0) wh[dig] = (uint16_t)(old + __popc(peers));
-    __syncwarp();
-    rank[i] = old + __popc(peers & lt);
-  }
-}
-
-// One stable LSD pass over (key, value) pairs for the kBits-bit digit at
-// `digit` (bits digit * kDigitBits ...), with decoupled look-back across
-// tiles.  Indices are 32-bit: the key count is below 2^31 (the C ABI's int
-// sizes).
-template <int kBits>
-__global__ void __launch_bounds__(kSortThreads, 2)
-    onesweep_kernel(int digit, SortBufs bufs, int64_t n64, uint64_t* __restrict__ status,
-                    BuildCtrl* __restrict__ ctrl, int flags)
-{
-  using L = SweepSmem<kBits>;
-  constexpr int kB = L::kB;
-  constexpr uint32_t kMask = (uint32_t)kB - 1u;
-  constexpr int kBPT = (kB + kSortThreads - 1) / kSortThreads;  // bins per thread
-  extern __shared__ __align__(16) unsigned char sweep_smem[];
-  uint32_t* s_key = (uint32_t*)(sweep_smem + L::kKeys);
-  uint32_t* s_val = (uint32_t*)(sweep_smem + L::kVals);
-  uint32_t* s_vin = (uint32_t*)(sweep_smem + L::kVin);
-  uint16_t* s_whist = (uint16_t*)(sweep_smem + L::kHist);
-  int* s_gbase = (int*)(sweep_smem + L::kGbase);
-  int* s_wsum = (int*)(sweep_smem + L::kWsum);
-  __shared__ int s_tile;
-
-  const int active = ctrl->active;
-  if (!((active >> digit) & 1)) return;
-  const int before = active & ((1 << digit) - 1);
-  const int parity = __popc(before) & 1;
-  const bool first = before == 0 && !(flags & kSortGivenValues);
-  const bool last = (active >> (digit + 1)) == 0 && !(flags & kSortKeepKeys);
-  const int shift = digit * kDigitBits;
-  const int n = (int)n64;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(&ctrl->tile_ctr[digit], 1);
-  for (int i = tid; i < kSortWarps * kB / 2; i += kSortThreads) ((uint32_t*)s_whist)[i] = 0;
-  if (kB < 2 && tid < kSortWarps) s_whist[tid] = 0;
-  __syncthreads();
-  const int tile = s_tile;
-  const int base = tile * kSortTile;
-  const int tile_n = min(kSortTile, n - base);
-  const uint32_t* __restrict__ src_k = bufs.keys[parity] + base;
-  const uint32_t* __restrict__ src_v = bufs.vals[parity] + base;
-  uint32_t* __restrict__ dst_k = bufs.keys[parity ^ 1];
-  uint32_t* __restrict__ dst_v = bufs.vals[parity ^ 1];
-  const int wbase = warp * 32 * kSortIpt + lane;  // this lane's first item in the tile
-
-  // the tile's incoming values land in shared memory while the keys are
-  // ranked (16-byte async copies; the tile start is 32 KiB-aligned)
-  if (L::kPrefetch && !first) {
-#pragma unroll
-    for (int c = tid; c < kSortTile / 4; c += kSortThreads) {
-      const int left = tile_n - 4 * c;
-      if (left > 0) {
-        const int bytes = min(left, 4) * 4;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(s_vin + 4 * c)),
-                     "l"(src_v + 4 * c), "r"(bytes)
-                     : "memory");
-      }
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  }
-
-  // load keys (warp-striped: item i of a lane is wbase + 32 i)
-  uint32_t key[kSortIpt];
-  uint32_t rank[kSortIpt];
-  uint16_t* wh = s_whist + warp * kB;
-  if (tile_n == kSortTile) {
-#pragma unroll
-    for (int i = 0; i < kSortIpt; i++) key[i] = src_k[wbase + 32 * i];
-    rank_keys<true, kBits>(key, rank, wh, wbase, tile_n, shift);
-  } else {
-#pragma unroll
-    for (int i = 0; i < kSortIpt; i++) {
-      const int j = wbase + 32 * i;
-      key[i] = j < tile_n ? src_k[j] : 0u;
-    }
-    rank_keys<false, kBits>(key, rank, wh, wbase, tile_n, shift);
-  }
-  __syncthreads();
-  // per owned bin: exclusive prefix over warps and the tile count
-  int cnt[kBPT];
-  int tsum = 0;
-#pragma unroll
-  for (int j = 0; j < kBPT; j++) {
-    const int b = tid * kBPT + j;
-    int run = 0;
-    if (b < kB) {
-#pragma unroll
-      for (int w = 0; w < kSortWarps; w++) {
-        const int c = (int)s_whist[w * kB + b];
-        s_whist[w * kB + b] = (uint16_t)run;
-        run += c;
-      }
-    }
-    cnt[j] = run;
-    tsum += run;
-  }
-  // exclusive scan of the per-thread bin sums over the CTA (bins in order)
-  int x = tsum;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) s_wsum[warp] = x;
-  // publish this tile's aggregate of every owned bin before waiting on
-  // predecessors (tile 0 publishes its inclusive count at once)
-#pragma unroll
-  for (int j = 0; j < kBPT; j++) {
-    const int b = tid * kBPT + j;
-    if (b < kB)
-      st_relaxed_u64(&status[(int64_t)tile * kB + b],
-                     (tile == 0 ? kFlagIncl : kFlagAgg) | (uint32_t)cnt[j]);
-  }
-  __syncthreads();
-  int binstart = x - tsum;
-  for (int w = 0; w < warp; w++) binstart += s_wsum[w];
-#pragma unroll
-  for (int j = 0; j < kBPT; j++) {
-    const int b = tid * kBPT + j;
-    if (b < kB) {
-      // fold the bin start into every warp's offset: one lookup per key later
-#pragma unroll
-      for (int w = 0; w < kSortWarps; w++)
-        s_whist[w * kB + b] = (uint16_t)(s_whist[w * kB + b] + binstart);
-      // decoupled look-back for bin b
-      int excl = 0;
-      if (tile > 0) {
-        int t = tile - 1;
-        uint32_t spins = 0;
-        while (true) {
-          const uint64_t v = ld_relaxed_u64(&status[(int64_t)t * kB + b]);
-          const uint64_t flag = v & (3ull << 62);
-          if (flag == 0) {
-            if (++spins > kSpinLimit || ld_relaxed_i32(&ctrl->error) != 0) {
-              raise_error(&ctrl->error, CRT_ERR_DEVICE_TIMEOUT);
-              break;
-            }
-            if (spins > 64) __nanosleep(64);
-            continue;
-          }
-          excl += (int)(uint32_t)v;
-          if (flag == kFlagIncl) break;
-          --t;
-        }
-        st_relaxed_u64(&status[(int64_t)tile * kB + b], kFlagIncl | (uint32_t)(excl + cnt[j]));
-      }
-      s_gbase[b] = ctrl->bucket_start[digit * kBins + b] + excl - binstart;
-    }
-    binstart += cnt[j];
-  }
-  if (L::kPrefetch && !first) asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
-
-  // stage (key, value) pairs in the order of their destination
-#pragma unroll
-  for (int i = 0; i < kSortIpt; i++) {
-    const int j = wbase + 32 * i;
-    const int pos = (int)(wh[(key[i] >> shift) & kMask] + rank[i]);
-    if (j < tile_n && (unsigned)pos < (unsigned)kSortTile) {  // pos < tile_n by construction
-      s_key[pos] = key[i];
-      if (first) {
-        s_val[pos] = (uint32_t)(base + j);
-      } else if (L::kPrefetch) {
-        s_val[pos] = s_vin[j];
-      } else {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(s_val + pos)),
-                     "l"(src_v + j)
-                     : "memory");
-      }
-    }
-  }
-  if (!L::kPrefetch && !first) {
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_all;" ::: "memory");
-  }
-  __syncthreads();
-  for (int j = tid; j < tile_n; j += kSortThreads) {
-    const uint32_t k = s_key[j];
-    const int dst = s_gbase[(k >> shift) & kMask] + j;
-    if ((uint32_t)dst < (uint32_t)n) {
-      // evict-first: a pass's output is read once, by the next pass, and
-      // the look-back status words and the next tiles' runs want L2
-      if (!last) __stcs(dst_k + dst, k);
-      __stcs(dst_v + dst, s_val[j]);
-    }
-  }
+  sort_plan(ctrl, n, kDigits);
 }
 
 // ---------------------------------------------------------------------------
@@ -522,7 +218,7 @@ __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs
                  int64_t parent_start, int64_t pos_base,
                  // leaf inputs/outputs
                  const uint32_t* __restrict__ vals0, const uint32_t* __restrict__ vals1,
-                 const BuildCtrl* __restrict__ ctrl, const Box32* __restrict__ aos,
+                 const SortCtrl* __restrict__ ctrl, const Box32* __restrict__ aos,
                  float* __restrict__ oxmin, float* __restrict__ oymin,
                  float* __restrict__ oxmax, float* __restrict__ oymax, int* __restrict__ oid,
                  // node arrays
@@ -631,57 +327,6 @@ int tree_levels(int64_t n, int fanout, std::vector<int64_t>& lv)
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-static int64_t sort_tiles(int64_t n) { return std::max<int64_t>(1, cdiv(n, kSortTile)); }
-
-// Look-back status words: one per (tile, bin) of every digit.
-static int64_t status_words_before(int digit, int64_t tiles)
-{
-  int64_t w = 0;
-  for (int d = 0; d < digit; d++) w += tiles << digit_bits(d);
-  return w;
-}
-
-size_t sort_zero_bytes(int64_t n)
-{
-  return sizeof(SortCtrl) + (size_t)kDigits * kBins * sizeof(uint32_t) +
-         (size_t)status_words_before(kDigits, sort_tiles(n)) * sizeof(uint64_t);
-}
-SortCtrl* sort_ctrl(void* zero_block) { return (SortCtrl*)zero_block; }
-uint32_t* sort_hist(void* zero_block) { return (uint32_t*)((char*)zero_block + sizeof(SortCtrl)); }
-static uint64_t* sort_status(void* zero_block)
-{
-  return (uint64_t*)((char*)zero_block + sizeof(SortCtrl) + (size_t)kDigits * kBins * sizeof(uint32_t));
-}
-
-template <int kBits>
-static void launch_pass(int d, SortBufs bufs, int64_t n, uint64_t* status, SortCtrl* ctrl,
-                        int flags, cudaStream_t stream)
-{
-  const size_t smem = SweepSmem<kBits>::kBytes;
-  cudaFuncSetAttribute(onesweep_kernel<kBits>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  onesweep_kernel<kBits><<<(unsigned)sort_tiles(n), kSortThreads, smem, stream>>>(d, bufs, n, status,
-                                                                                  ctrl, flags);
-}
-
-void sort_passes(SortBufs bufs, int64_t n, void* zero_block, cudaStream_t stream, int flags)
-{
-  const int64_t ntiles = sort_tiles(n);
-  SortCtrl* ctrl = sort_ctrl(zero_block);
-  plan_kernel<<<1, 32 * kDigits, 0, stream>>>(sort_hist(zero_block), n, ctrl);
-  for (int d = 0; d < kDigits; d++) {
-    ProfScope ps("sort_pass", stream);
-    uint64_t* status = sort_status(zero_block) + status_words_before(d, ntiles);
-    switch (digit_bits(d)) {
-      case 10: launch_pass<10>(d, bufs, n, status, ctrl, flags, stream); break;
-      case 8: launch_pass<8>(d, bufs, n, status, ctrl, flags, stream); break;
-      case 2: launch_pass<2>(d, bufs, n, status, ctrl, flags, stream); break;
-      default: launch_pass<kDigitBits>(d, bufs, n, status, ctrl, flags, stream); break;
-    }
-  }
-  CRT_LAUNCHED(1 + kDigits);
-}
-
 // Builds the tree of `n` boxes.  in_* may alias out_* (in-place build).
 // Node arrays must hold R_sz entries.  Synchronises `stream` at the end and
 // reports device-side errors.
@@ -712,13 +357,13 @@ int build_tree(const float* in_xmin, const float* in_ymin, const float* in_xmax,
     return fail(CRT_ERR_OOM, "build: scratch allocation failed");
   }
   size_t off = (zero_bytes + 255) / 256 * 256;
-  BuildCtrl* ctrl = sort_ctrl(scratch);
-  uint32_t* hist = sort_hist(scratch);
-  SortBufs bufs;
-  bufs.keys[0] = (uint32_t*)(scratch + off); off += kv_bytes;
-  bufs.keys[1] = (uint32_t*)(scratch + off); off += kv_bytes;
-  bufs.vals[0] = (uint32_t*)(scratch + off); off += kv_bytes;
-  bufs.vals[1] = (uint32_t*)(scratch + off); off += kv_bytes;
+  SortCtrl* ctrl = sort_ctrl(scratch);
+  SortCols cols{};
+  cols.key[0] = (uint32_t*)(scratch + off); off += kv_bytes;
+  cols.key[1] = (uint32_t*)(scratch + off); off += kv_bytes;
+  cols.val[0] = (uint32_t*)(scratch + off); off += kv_bytes;
+  cols.val[1] = (uint32_t*)(scratch + off); off += kv_bytes;
+  cols.drop_keys = true;
   Box32* aos = (Box32*)(scratch + off);
 
   int rc = CRT_OK;
@@ -733,14 +378,14 @@ int build_tree(const float* in_xmin, const float* in_ymin, const float* in_xmax,
     {
     ProfScope ps("encode", stream);
     if (vec)
-      encode_kernel<true><<<grid, kEncThreads, 0, stream>>>(bin, n, bufs.keys[0], bufs.vals[0],
-                                                            aos, hist);
+      encode_kernel<true><<<grid, kEncThreads, 0, stream>>>(bin, n, cols.key[0], cols.val[0], aos,
+                                                            ctrl);
     else
-      encode_kernel<false><<<grid, kEncThreads, 0, stream>>>(bin, n, bufs.keys[0], bufs.vals[0],
-                                                             aos, hist);
+      encode_kernel<false><<<grid, kEncThreads, 0, stream>>>(bin, n, cols.key[0], cols.val[0], aos,
+                                                             ctrl);
     }
     CRT_LAUNCHED(1);
-    sort_passes(bufs, n, scratch, stream, kSortGivenValues);
+    sort_passes(cols, n, kDigits, scratch, stream);
 
     // leaf-parent level
     int64_t parent_start = rsz;
@@ -753,7 +398,7 @@ int build_tree(const float* in_xmin, const float* in_ymin, const float* in_xmax,
       ProfScope ps("level", stream);
       if (l == 0)
         level_kernel<true><<<g, kLevelThreads, 0, stream>>>(
-            npc, fanout, nchild, np, parent_start, rsz, bufs.vals[0], bufs.vals[1], ctrl, aos,
+            npc, fanout, nchild, np, parent_start, rsz, cols.val[0], cols.val[1], ctrl, aos,
             out_xmin, out_ymin, out_xmax, out_ymax, out_id, nxmin, nymin, nxmax, nymax, npos,
             nlen, 0);
       else

@@ -10,43 +10,85 @@
 
 namespace crt {
 
-// keys = key_src ^ 0x80000000 (signed order as unsigned), vals = val_src, and
-// the four digit histograms of the keys.
-__global__ void canon_stage_kernel(const int32_t* __restrict__ key_src,
-                                   const int32_t* __restrict__ val_src, int64_t n,
-                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                   uint32_t* __restrict__ hist)
+// Digit histograms of both columns (signed order: the top digit's sign bit
+// flipped), four of the box ids and four of the windows; the last CTA plans
+// the passes.  The histograms do not depend on the order of the pairs, so one
+// read serves all eight passes.
+__global__ void __launch_bounds__(256)
+    canon_hist_kernel(const int32_t* __restrict__ fid, const int32_t* __restrict__ tid, int64_t n,
+                      SortCtrl* __restrict__ ctrl)
 {
-  __shared__ uint32_t sh[kDigits][kBins];
-  for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) (&sh[0][0])[i] = 0;
+  __shared__ uint32_t sh[2 * kDigits][kBins];
+  for (int i = threadIdx.x; i < 2 * kDigits * kBins; i += blockDim.x) (&sh[0][0])[i] = 0;
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const uint32_t k = (uint32_t)key_src[i] ^ 0x80000000u;
-    keys[i] = k;
-    vals[i] = (uint32_t)val_src[i];
+    const uint32_t k = (uint32_t)fid[i] ^ 0x80000000u, w = (uint32_t)tid[i] ^ 0x80000000u;
 #pragma unroll
-    for (int d = 0; d < kDigits; d++) atomicAdd(&sh[d][key_digit(k, d)], 1u);
+    for (int d = 0; d < kDigits; d++) {
+      atomicAdd(&sh[d][key_digit(k, d)], 1u);
+      atomicAdd(&sh[kDigits + d][key_digit(w, d)], 1u);
+    }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) {
+  for (int i = threadIdx.x; i < 2 * kDigits * kBins; i += blockDim.x) {
     const uint32_t v = (&sh[0][0])[i];
-    if (v) atomicAdd(&hist[i], v);
+    if (v) atomicAdd(&ctrl->hist[i], v);
+  }
+  sort_plan(ctrl, n, 2 * kDigits);
+}
+
+// Short lists: one CTA sorts the pairs in shared memory as 64-bit keys (window
+// above, box id below, sign bits flipped) with a bitonic network (Batcher,
+// "Sorting networks and their applications", 1968).  Equal keys are equal
+// pairs, so stability does not matter.  Thread t compares elements i and i + j
+// with i = 2t - (t mod j): for j <= 32 a warp stays inside its own 64
+// elements and needs no block barrier.  A call with 244 pairs takes 20 us;
+// its eight radix passes, nearly all launch latency, took 64 us.
+constexpr int kCanonSmall = 8192;
+
+__global__ void __launch_bounds__(1024)
+    canon_small_kernel(int32_t* __restrict__ fid, int32_t* __restrict__ tid, int n, int size)
+{
+  extern __shared__ unsigned long long s_pair[];
+  for (int i = threadIdx.x; i < size; i += blockDim.x)
+    s_pair[i] = i < n ? (unsigned long long)((uint32_t)tid[i] ^ 0x80000000u) << 32 |
+                            ((uint32_t)fid[i] ^ 0x80000000u)
+                      : ~0ull;
+  __syncthreads();
+  for (int k = 2; k <= size; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      for (int t = threadIdx.x; t < size / 2; t += blockDim.x) {
+        const int i = 2 * t - (t & (j - 1));
+        const unsigned long long a = s_pair[i], b = s_pair[i + j];
+        if ((a > b) == ((i & k) == 0)) {
+          s_pair[i] = b;
+          s_pair[i + j] = a;
+        }
+      }
+      // the next step's elements: this warp's own (j <= 32), or any warp's
+      if (j > 32 || (j == 1 && k >= 64)) __syncthreads();
+      else __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const unsigned long long v = s_pair[i];
+    tid[i] = (int32_t)((uint32_t)(v >> 32) ^ 0x80000000u);
+    fid[i] = (int32_t)((uint32_t)v ^ 0x80000000u);
   }
 }
 
-// Writes the sorted (key, value) pairs back: key_dst = key ^ 0x80000000,
-// val_dst = value, from the buffers the passes left them in.
-__global__ void canon_unstage_kernel(SortBufs bufs, const SortCtrl* __restrict__ ctrl, int64_t n,
-                                     int32_t* __restrict__ key_dst, int32_t* __restrict__ val_dst)
+// A sort of one pass ends in the scratch buffer: back to the caller's arrays.
+__global__ void canon_copy_kernel(const SortCtrl* __restrict__ ctrl, int64_t n,
+                                  const uint32_t* __restrict__ sf, const uint32_t* __restrict__ st,
+                                  uint32_t* __restrict__ fid, uint32_t* __restrict__ tid)
 {
-  const int p = ctrl->n_active & 1;
-  const uint32_t* __restrict__ keys = bufs.keys[p];
-  const uint32_t* __restrict__ vals = bufs.vals[p];
+  if (ctrl->n_active != 1) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    key_dst[i] = (int32_t)(keys[i] ^ 0x80000000u);
-    val_dst[i] = (int32_t)vals[i];
+    fid[i] = sf[i];
+    tid[i] = st[i];
   }
 }
 
@@ -56,32 +98,47 @@ int pairs_canonicalize(int32_t* fid, int32_t* tid, int64_t n, cudaStream_t strea
   if (n <= 1) return CRT_OK;
   if (n > INT32_MAX)
     return fail(CRT_ERR_NOT_SUPPORTED, "canonicalize: at most INT32_MAX pairs per call");
-  const size_t zero = (sort_zero_bytes(n) + 255) / 256 * 256;
+  if (n <= kCanonSmall) {
+    int size = 64;
+    while (size < n) size <<= 1;
+    const size_t smem = sizeof(unsigned long long) * (size_t)size;
+    cudaFuncSetAttribute(canon_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(sizeof(unsigned long long) * kCanonSmall));
+    canon_small_kernel<<<1, std::min(1024, size / 2), smem, stream>>>(fid, tid, (int)n, size);
+    CRT_LAUNCHED(1);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    return e == cudaSuccess ? CRT_OK : cuda_fail(e, "canonicalize");
+  }
+  const size_t zero = (sort_zero_bytes(n, 2 * kDigits) + 255) / 256 * 256;
   const size_t kv = ((size_t)n * 4 + 255) / 256 * 256;
   char* scr = nullptr;
   if (cudaMallocAsync((void**)&scr, zero + 4 * kv, stream) != cudaSuccess) {
     cudaGetLastError();
     return fail(CRT_ERR_OOM, "canonicalize: scratch allocation failed");
   }
-  SortBufs bufs;
-  bufs.keys[0] = (uint32_t*)(scr + zero);
-  bufs.keys[1] = (uint32_t*)(scr + zero + kv);
-  bufs.vals[0] = (uint32_t*)(scr + zero + 2 * kv);
-  bufs.vals[1] = (uint32_t*)(scr + zero + 3 * kv);
-  const int grid = (int)std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 8);
-  // by box id (carrying the window), then stably by window (carrying the box id)
-  for (int round = 0; round < 2; round++) {
-    int32_t* key_src = round == 0 ? fid : tid;
-    int32_t* val_src = round == 0 ? tid : fid;
-    cudaMemsetAsync(scr, 0, sort_zero_bytes(n), stream);
-    canon_stage_kernel<<<grid, 256, 0, stream>>>(key_src, val_src, n, bufs.keys[0], bufs.vals[0],
-                                                 sort_hist(scr));
-    sort_passes(bufs, n, scr, stream, kSortGivenValues | kSortKeepKeys);
-    canon_unstage_kernel<<<grid, 256, 0, stream>>>(bufs, sort_ctrl(scr), n, key_src, val_src);
-    CRT_LAUNCHED(2);
+  // by box id (carrying the window), then stably by window (carrying the box
+  // id): passes 4-7 take the other column's digits.  The first pass reads the
+  // caller's arrays and the last one writes them.
+  SortCols cols{};
+  cols.key[0] = (uint32_t*)fid;
+  cols.val[0] = (uint32_t*)tid;
+  for (int b = 0; b < 2; b++) {
+    cols.key[1 + b] = (uint32_t*)(scr + zero + 2 * b * kv);
+    cols.val[1 + b] = (uint32_t*)(scr + zero + (2 * b + 1) * kv);
   }
+  cols.flip = 0x80000000u;
+  cols.home = true;
+  SortCtrl* ctrl = sort_ctrl(scr);
+  const int grid = (int)std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 8);
+  cudaMemsetAsync(scr, 0, sort_zero_bytes(n, 2 * kDigits), stream);
+  canon_hist_kernel<<<grid, 256, 0, stream>>>(fid, tid, n, ctrl);
+  sort_passes(cols, n, 2 * kDigits, scr, stream);
+  canon_copy_kernel<<<grid, 256, 0, stream>>>(ctrl, n, cols.key[1], cols.val[1], cols.key[0],
+                                              cols.val[0]);
+  CRT_LAUNCHED(2);
   int dev_err = 0;
-  cudaMemcpyAsync(&dev_err, &sort_ctrl(scr)->error, sizeof(int), cudaMemcpyDeviceToHost, stream);
+  cudaMemcpyAsync(&dev_err, &ctrl->error, sizeof(int), cudaMemcpyDeviceToHost, stream);
   cudaFreeAsync(scr, stream);
   cudaError_t e = cudaStreamSynchronize(stream);
   if (e != cudaSuccess) return cuda_fail(e, "canonicalize");

@@ -7,65 +7,9 @@
 #include <vector>
 
 #include "common.cuh"
+#include "sort.cuh"
 
 namespace crt {
-
-// Radix-sort scratch shared by the box build and the window ordering.
-struct SortBufs {
-  uint32_t* keys[2];
-  uint32_t* vals[2];
-};
-
-// Radix digits of the 32-bit sort keys: kDigits digits of kDigitBits bits
-// from the least significant end, the last one narrower when kDigitBits does
-// not divide 32.  Histograms and bucket starts keep kBins entries per digit.
-// 8-bit digits (four passes, uniform digits skipped) measured faster on a
-// B200 than 10 + 10 + 10 + 2 (three passes for 30-bit Morton keys): 2.74
-// against 3.43 ms for 100M keys, the 1024-bin passes paying more for ranking,
-// bin scans and look-back than the fourth pass costs.
-#ifndef CRT_SORT_DIGIT_BITS
-#define CRT_SORT_DIGIT_BITS 8
-#endif
-constexpr int kDigitBits = CRT_SORT_DIGIT_BITS;
-constexpr int kBins = 1 << kDigitBits;
-constexpr int kDigits = (32 + kDigitBits - 1) / kDigitBits;
-static_assert(kDigits == 4, "four digit passes at most");
-constexpr int kSortTile = 8192;
-
-__host__ __device__ constexpr int digit_bits(int d)
-{
-  return 32 - d * kDigitBits < kDigitBits ? 32 - d * kDigitBits : kDigitBits;
-}
-__device__ __forceinline__ uint32_t key_digit(uint32_t k, int d)
-{
-  return (k >> (d * kDigitBits)) & ((1u << digit_bits(d)) - 1u);
-}
-
-// Control block of one sort (int32 words, zero-initialised by the caller).
-struct SortCtrl {
-  int tile_ctr[4];  // per pass: next tile index
-  int error;        // first device error
-  int active;       // bit d: digit d is non-uniform
-  int n_active;     // number of active passes: the order is in vals[n_active & 1]
-  int pad[9];
-  int bucket_start[kDigits * kBins];
-};
-
-// Bytes of zero-initialised state a sort of n keys needs: SortCtrl, the
-// digit histograms (kDigits x kBins words, filled by the caller's key kernel
-// with key_digit) and the look-back status words (in that order).
-size_t sort_zero_bytes(int64_t n);
-// Enqueues plan + four onesweep passes; keys must be in bufs.keys[0] and the
-// histograms filled.  The sorted positions end in bufs.vals[n_active & 1]
-// (identity when no pass is active).
-// flags: kSortGivenValues -- the values are in bufs.vals[0] (otherwise the
-// first pass makes them: positions 0..n-1); kSortKeepKeys -- the sorted keys
-// are kept too, in bufs.keys[n_active & 1] (otherwise the last pass drops them).
-constexpr int kSortGivenValues = 1;
-constexpr int kSortKeepKeys = 2;
-void sort_passes(SortBufs bufs, int64_t n, void* zero_block, cudaStream_t stream, int flags = 0);
-uint32_t* sort_hist(void* zero_block);
-SortCtrl* sort_ctrl(void* zero_block);
 
 int tree_levels(int64_t n, int fanout, std::vector<int64_t>& lv);
 

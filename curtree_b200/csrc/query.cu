@@ -799,7 +799,7 @@ __global__ void __launch_bounds__(256)
 
 // Window keys (same Morton key as the boxes) and digit histograms.
 __global__ void window_key_kernel(WindowView W, uint32_t* __restrict__ keys,
-                                  uint32_t* __restrict__ hist)
+                                  SortCtrl* __restrict__ ctrl)
 {
   __shared__ uint32_t sh[kDigits][kBins];
   for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) (&sh[0][0])[i] = 0;
@@ -814,8 +814,9 @@ __global__ void window_key_kernel(WindowView W, uint32_t* __restrict__ keys,
   __syncthreads();
   for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) {
     uint32_t v = (&sh[0][0])[i];
-    if (v) atomicAdd(&hist[i], v);
+    if (v) atomicAdd(&ctrl->hist[i], v);
   }
+  sort_plan(ctrl, W.n, kDigits);
 }
 
 __global__ void set_nq_kernel(QueryCounters* ctr, long long nq) { ctr->nq = (unsigned long long)nq; }
@@ -1010,7 +1011,7 @@ struct PersistScratch {
   Hole* sorted;
   long long* cum;
   void* sort_zero;
-  SortBufs bufs;
+  SortCols cols;
   long long max_holes;
   JobQueue* jobs;
   size_t bytes;
@@ -1036,13 +1037,15 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
   S.cum = (long long*)(base + off); off += al(sizeof(long long) * (max_holes + 1));
   S.jobs = (JobQueue*)(base + off); off += al(kJobQueueBytes);
   S.sort_zero = nullptr;
+  S.cols = SortCols{};
   if (sort) {
     S.sort_zero = base + off; off += al(sort_zero_bytes(max_nq));
     size_t kv = al(4 * (size_t)std::max<int64_t>(max_nq, 1));
-    S.bufs.keys[0] = (uint32_t*)(base + off); off += kv;
-    S.bufs.keys[1] = (uint32_t*)(base + off); off += kv;
-    S.bufs.vals[0] = (uint32_t*)(base + off); off += kv;
-    S.bufs.vals[1] = (uint32_t*)(base + off); off += kv;
+    S.cols.key[0] = (uint32_t*)(base + off); off += kv;
+    S.cols.key[1] = (uint32_t*)(base + off); off += kv;
+    S.cols.val[0] = (uint32_t*)(base + off); off += kv;
+    S.cols.val[1] = (uint32_t*)(base + off); off += kv;
+    S.cols.make_values = S.cols.drop_keys = true;
   }
   S.max_holes = max_holes;
   S.bytes = off;
@@ -1062,8 +1065,8 @@ static void enqueue_pre(const WindowView& W, int64_t max_nq, const PersistScratc
     const int sms = sm_count();
     cudaMemsetAsync(S.sort_zero, 0, sort_zero_bytes(max_nq), stream);
     int g = (int)std::min<int64_t>(cdiv(max_nq, 256), (int64_t)sms * 4);
-    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, S.bufs.keys[0], sort_hist(S.sort_zero));
-    sort_passes(S.bufs, W.n, S.sort_zero, stream);
+    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, S.cols.key[0], sort_ctrl(S.sort_zero));
+    sort_passes(S.cols, W.n, kDigits, S.sort_zero, stream);
     CRT_LAUNCHED(1);
   }
 }
@@ -1087,8 +1090,8 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
   PersistParams& P = L.P;
   P.T = T;
   P.W = W;
-  P.order0 = S.bufs.vals[0];
-  P.order1 = S.bufs.vals[1];
+  P.order0 = S.cols.val[0];
+  P.order1 = S.cols.val[1];
   P.sort_ctrl = sort ? sort_ctrl(S.sort_zero) : nullptr;
   P.K = sh.K;
   P.stack_cap = sh.stack_cap;
@@ -1576,9 +1579,9 @@ int plan_launch(void* hp, cudaStream_t stream)
     e = cudaGraphLaunch(p->exec, stream);
   }
   if (e != cudaSuccess) return cuda_fail(e, "plan_launch");
-  // window keys, sort plan, four sort passes; the traversal; hole sort,
+  // window keys and four sort passes; the traversal; hole sort,
   // prefix and compaction
-  CRT_LAUNCHED((p->sort ? 6 : 0) + 1 + 3);
+  CRT_LAUNCHED((p->sort ? 5 : 0) + 1 + 3);
   return CRT_OK;
 }
 

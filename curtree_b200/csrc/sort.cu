@@ -1,0 +1,330 @@
+// Stable LSD radix sort of (key, value) pairs of 32-bit words, shared by the
+// bulk load (Morton keys), the window ordering and the canonical pair order.
+// The caller's key kernel fills the digit histograms and its last CTA plans
+// the passes (sort_plan, sort.cuh); every pass then is one launch that reads
+// and writes the pairs once, with decoupled look-back across tiles.
+//
+// A pass is bound by instruction issue (the in-warp ranking) and by the chain
+// ticket -> keys -> ranks -> bin scan -> look-back -> stores inside a tile,
+// not by DRAM: 100M pairs take 0.58 ms per pass, 2.8 TB/s.  What shortened the
+// chain (0.67 ms before): the values go through registers, on their way while
+// the bins are scanned, instead of through a third shared-memory buffer; the
+// look-back comes after the staging, when the predecessors have mostly
+// published; no second launch to plan the passes.  CTAs that stay resident
+// and fetch their next tile's ticket and keys early measured slower (2.94
+// against 2.30 ms): a claimed tile waits for its CTA, and every successor's
+// look-back waits for that tile.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "profile.h"
+#include "sort.cuh"
+
+namespace crt {
+
+constexpr uint64_t kFlagAgg = 1ull << 62;
+constexpr uint64_t kFlagIncl = 2ull << 62;
+constexpr uint64_t kFlagMask = 3ull << 62;
+// Predecessors a look-back reads per round trip (100M keys, four passes: 1 2.33,
+// 2 2.32, 4 2.30, 8 2.42 ms).
+constexpr int kLook = 4;
+
+// Lanes of the warp whose value equals this lane's (v < 2^kBits), from one
+// ballot per bit; on this part it issues faster than __match_any_sync
+// (measured over the four 8-bit passes of a 100M-key build: 3.7 ms against
+// 4.3 ms).
+template <int kBits>
+__device__ __forceinline__ uint32_t peer_mask(uint32_t v)
+{
+  uint32_t peers = 0xffffffffu;
+#pragma unroll
+  for (int b = 0; b < kBits; b++) {
+    const bool bit = (v >> b) & 1u;
+    const uint32_t bal = __ballot_sync(0xffffffffu, bit);
+    peers &= bit ? bal : ~bal;
+  }
+  return peers;
+}
+
+// Shared memory of one pass: keys and values staged in destination order, the
+// per-warp digit counters (16-bit: at most a tile's keys), the bins' global
+// offsets and the warp sums of the bin scan.
+template <int kThreads, int kIpt>
+struct SweepSmem {
+  static constexpr int kTile = kThreads * kIpt;
+  static constexpr int kWarps = kThreads / 32;
+  static constexpr size_t kKeys = 0;
+  static constexpr size_t kVals = kKeys + 4 * (size_t)kTile;
+  static constexpr size_t kHist = kVals + 4 * (size_t)kTile;
+  static constexpr size_t kGbase = kHist + 2 * (size_t)kWarps * kBins;
+  static constexpr size_t kWsum = kGbase + 4 * (size_t)kBins;
+  static constexpr size_t kBytes = kWsum + 4 * 32;
+};
+
+// Ranks this thread's keys inside its warp, stably (rounds in order, lanes in
+// order), two 16-bit ranks per word.  kFull: every item of the tile is valid
+// (no bounds checks); otherwise invalid items take digit 256.
+template <bool kFull, int kIpt>
+__device__ __forceinline__ void rank_keys(const uint32_t (&key)[kIpt], uint32_t (&rank)[kIpt / 2],
+                                          uint16_t* wh, int wbase, int tile_n, int shift,
+                                          uint32_t flip)
+{
+  const uint32_t lt = lanemask_lt();
+#pragma unroll
+  for (int i = 0; i < kIpt; i++) {
+    const bool v = kFull || wbase + 32 * i < tile_n;
+    const uint32_t dig = v ? ((key[i] ^ flip) >> shift) & 255u : 256u;
+    const uint32_t peers = kFull ? peer_mask<8>(dig) : peer_mask<9>(dig);
+    const uint32_t old = v ? wh[dig] : 0u;
+    __syncwarp();
+    if (v && (peers & lt) == 0) wh[dig] = (uint16_t)(old + __popc(peers));
+    __syncwarp();
+    const uint32_t r = old + __popc(peers & lt);
+    if (i & 1) rank[i / 2] |= r << 16;
+    else rank[i / 2] = r;
+  }
+}
+
+// One stable pass over the 8-bit digit `digit` (digits 0-3 of the key column;
+// 4-7: of the value column, the columns then change roles).  A CTA takes one
+// tile, in order from a ticket.  Indices are 32-bit: the pair count is below
+// 2^31 (the C ABI's int sizes).
+template <int kThreads, int kIpt, int kMinBlocks>
+__global__ void __launch_bounds__(kThreads, kMinBlocks)
+    sweep_kernel(int digit, SortCols cols, int64_t n64, uint64_t* __restrict__ status,
+                 SortCtrl* __restrict__ ctrl)
+{
+  using L = SweepSmem<kThreads, kIpt>;
+  constexpr int kTile = L::kTile;
+  constexpr int kWarps = L::kWarps;
+  static_assert(kThreads >= kBins, "one thread per bin");
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  uint32_t* s_key = (uint32_t*)(sweep_smem + L::kKeys);
+  uint32_t* s_val = (uint32_t*)(sweep_smem + L::kVals);
+  uint16_t* s_whist = (uint16_t*)(sweep_smem + L::kHist);
+  int* s_gbase = (int*)(sweep_smem + L::kGbase);
+  int* s_wsum = (int*)(sweep_smem + L::kWsum);
+  __shared__ int s_tile, s_stop;
+
+  const int active = ctrl->active;
+  if (!((active >> digit) & 1)) return;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    s_tile = atomicAdd(&ctrl->tile_ctr[digit], 1);
+    s_stop = 0;
+  }
+  for (int i = tid; i < kWarps * kBins / 2; i += kThreads) ((uint32_t*)s_whist)[i] = 0;
+  const int step = __popc(active & ((1 << digit) - 1));  // active passes before this one
+  const bool last = (active >> (digit + 1)) == 0;
+  const int src = cols.src(step), dst = cols.dst(step, last);
+  const bool swap = digit >= 4;
+  const bool make_vals = step == 0 && cols.make_values;
+  const bool drop_keys = last && cols.drop_keys;
+  const int shift = 8 * (digit & 3);
+  const uint32_t flip = cols.flip;
+  const int n = (int)n64;
+  const uint32_t* __restrict__ src_k = swap ? cols.vals(src) : cols.keys(src);
+  const uint32_t* __restrict__ src_v = swap ? cols.keys(src) : cols.vals(src);
+  uint32_t* __restrict__ dst_k = swap ? cols.vals(dst) : cols.keys(dst);
+  uint32_t* __restrict__ dst_v = swap ? cols.keys(dst) : cols.vals(dst);
+  const int bucket = tid < kBins ? ctrl->bucket_start[digit * kBins + tid] : 0;
+  const int wbase = warp * 32 * kIpt + lane;  // this lane's first item in a tile
+  uint16_t* wh = s_whist + warp * kBins;
+  __syncthreads();
+  const int tile = s_tile;
+  const int base = tile * kTile;
+  const int tile_n = min(kTile, n - base);
+  const bool full = tile_n == kTile;
+
+  // keys (warp-striped: item i of a lane is wbase + 32 i), their ranks, and
+  // the values on their way while the bins are scanned
+  uint32_t key[kIpt], rank[kIpt / 2], val[kIpt];
+  if (full) {
+#pragma unroll
+    for (int i = 0; i < kIpt; i++) key[i] = src_k[base + wbase + 32 * i];
+    rank_keys<true, kIpt>(key, rank, wh, wbase, tile_n, shift, flip);
+#pragma unroll
+    for (int i = 0; i < kIpt; i++)
+      val[i] = make_vals ? (uint32_t)(base + wbase + 32 * i) : src_v[base + wbase + 32 * i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < kIpt; i++) {
+      const int j = wbase + 32 * i;
+      key[i] = j < tile_n ? src_k[base + j] : 0u;
+    }
+    rank_keys<false, kIpt>(key, rank, wh, wbase, tile_n, shift, flip);
+#pragma unroll
+    for (int i = 0; i < kIpt; i++) {
+      const int j = wbase + 32 * i;
+      val[i] = make_vals ? (uint32_t)(base + j) : (j < tile_n ? src_v[base + j] : 0u);
+    }
+  }
+  __syncthreads();
+  // bin b = tid: counts of every warp, the tile's count, exclusive scan over
+  // the bins; the tile's aggregate is published before anything waits
+  uint32_t cnt[kWarps / 2];  // two 16-bit counts per word
+  int total = 0, x = 0;
+  if (tid < kBins) {
+#pragma unroll
+    for (int w = 0; w < kWarps; w += 2) {
+      const uint32_t a = s_whist[w * kBins + tid], b = s_whist[(w + 1) * kBins + tid];
+      cnt[w / 2] = a | b << 16;
+      total += (int)(a + b);
+    }
+    st_relaxed_u64(&status[(int64_t)tile * kBins + tid],
+                   (tile == 0 ? kFlagIncl : kFlagAgg) | (uint32_t)total);
+    x = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) s_wsum[warp] = x;
+  }
+  __syncthreads();
+  int binstart = x - total;
+  if (tid < kBins) {
+    for (int w = 0; w < warp; w++) binstart += s_wsum[w];
+    int off = binstart;
+#pragma unroll
+    for (int w = 0; w < kWarps; w += 2) {
+      s_whist[w * kBins + tid] = (uint16_t)off;
+      off += (int)(cnt[w / 2] & 0xFFFFu);
+      s_whist[(w + 1) * kBins + tid] = (uint16_t)off;
+      off += (int)(cnt[w / 2] >> 16);
+    }
+  }
+  __syncthreads();
+  // stage the pairs in the order of their destination
+#pragma unroll
+  for (int i = 0; i < kIpt; i++) {
+    const uint32_t r = i & 1 ? rank[i / 2] >> 16 : rank[i / 2] & 0xFFFFu;
+    const int pos = (int)(wh[((key[i] ^ flip) >> shift) & 255u] + r);
+    if (full || wbase + 32 * i < tile_n) {
+      s_key[pos] = key[i];
+      s_val[pos] = val[i];
+    }
+  }
+  // decoupled look-back for bin b = tid, kLook predecessors per round trip
+  if (tid < kBins) {
+    int excl = 0;
+    if (tile > 0) {
+      int t = tile - 1;
+      uint32_t spins = 0;
+      bool found = false;
+      while (!found) {
+        uint64_t v[kLook];
+#pragma unroll
+        for (int u = 0; u < kLook; u++)
+          v[u] = t - u >= 0 ? ld_relaxed_u64(&status[(int64_t)(t - u) * kBins + tid]) : kFlagIncl;
+        int used = 0;
+        bool open = true;
+#pragma unroll
+        for (int u = 0; u < kLook; u++) {
+          open = open && (v[u] & kFlagMask) != 0;
+          if (open) {
+            excl += (int)(uint32_t)v[u];
+            used++;
+            if ((v[u] & kFlagMask) == kFlagIncl) {
+              found = true;
+              open = false;
+            }
+          }
+        }
+        t -= used;
+        if (!found && used == 0) {
+          if (++spins > kSpinLimit || ld_relaxed_i32(&ctrl->error) != 0) {
+            raise_error(&ctrl->error, CRT_ERR_DEVICE_TIMEOUT);
+            s_stop = 1;  // nothing of this tile is written
+            break;
+          }
+          if (spins > 64) __nanosleep(64);
+        }
+      }
+      if (found)
+        st_relaxed_u64(&status[(int64_t)tile * kBins + tid], kFlagIncl | (uint32_t)(excl + total));
+    }
+    s_gbase[tid] = bucket + excl - binstart;
+  }
+  __syncthreads();
+  if (s_stop) return;
+#pragma unroll
+  for (int i = 0; i < kIpt; i++) {
+    const int j = tid + i * kThreads;
+    if (full || j < tile_n) {
+      const uint32_t k = s_key[j];
+      const int d = s_gbase[((k ^ flip) >> shift) & 255u] + j;
+      // evict-first: a pass's output is read once, by the next pass, and
+      // the look-back status words and the next tiles' runs want L2
+      if (!drop_keys) __stcs(dst_k + d, k);
+      __stcs(dst_v + d, s_val[j]);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+struct SweepShape {
+  int threads;
+  int tile;
+  size_t smem;
+  const void* fn;
+};
+
+#define CRT_SHAPE(T, I, B) {T, (T) * (I), SweepSmem<T, I>::kBytes, (const void*)sweep_kernel<T, I, B>}
+// Tile shapes by pair count: {most pairs, shape}.  A tile's fixed cost (ticket,
+// bin scan, look-back) is a few microseconds whatever its size, so large sorts
+// want large tiles; small ones want enough tiles to use the SMs.  Sort of a
+// build (four passes, us with event overhead), by tile size:
+//   pairs   1024   4096   6144   8192
+//    20k      39     48     50     54
+//   200k      52     51     59     59
+//     1M     103     70     75     66
+//     3M     239    135    123    139
+//    10M     704    323    290    292
+//   100M    6717   2624   2361   2300
+// (1M: one tile of 8192 per SM, a single wave.)
+static const struct {
+  int64_t most;
+  SweepShape shape;
+} kShapes[] = {
+    {1 << 16, CRT_SHAPE(256, 4, 4)},
+    {3 << 18, CRT_SHAPE(256, 16, 4)},
+    {148 * 8192, CRT_SHAPE(512, 16, 2)},
+    {10'000'000, CRT_SHAPE(384, 16, 3)},
+    {INT64_MAX, CRT_SHAPE(512, 16, 2)},
+};
+
+static const SweepShape& shape_for(int64_t n)
+{
+  int i = 0;
+  while (n > kShapes[i].most) i++;
+  return kShapes[i].shape;
+}
+
+static int64_t sort_tiles(int64_t n) { return std::max<int64_t>(1, cdiv(n, shape_for(n).tile)); }
+
+size_t sort_zero_bytes(int64_t n, int digits)
+{
+  return sizeof(SortCtrl) + (size_t)digits * sort_tiles(n) * kBins * sizeof(uint64_t);
+}
+
+void sort_passes(const SortCols& cols, int64_t n, int digits, void* zero_block, cudaStream_t stream)
+{
+  const SweepShape& S = shape_for(n);
+  const int64_t tiles = sort_tiles(n);
+  SortCtrl* ctrl = sort_ctrl(zero_block);
+  cudaFuncSetAttribute(S.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem);
+  for (int d = 0; d < digits; d++) {
+    ProfScope ps("sort_pass", stream);
+    uint64_t* status = (uint64_t*)(ctrl + 1) + (size_t)d * tiles * kBins;
+    SortCols c = cols;
+    void* args[] = {&d, &c, &n, &status, &ctrl};
+    cudaLaunchKernel(S.fn, dim3((unsigned)tiles), dim3(S.threads), args, S.smem, stream);
+  }
+  CRT_LAUNCHED(digits);
+}
+
+}  // namespace crt
