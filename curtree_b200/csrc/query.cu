@@ -26,6 +26,10 @@
 //               4096-slot chunks a warp reserves with one atomic, and a
 //               compaction pass moves the tail of the array into the unused
 //               ends of each warp's last chunk so the output is dense.
+//               On sorted windows over packed trees the windows are classed by
+//               the boxes they can be expected to meet: huge ones are shared
+//               by several warps, small ones go to a kernel that takes 32
+//               neighbours per warp (small_windows_kernel).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -42,7 +46,10 @@ namespace crt {
 
 // Device-side counters of one query (int64 words; zeroed before a launch).
 struct QueryCounters {
-  unsigned long long ticket;  // next window (persistent)
+  unsigned long long ticket;  // next large window (persistent)
+  unsigned long long small_ticket;  // next small window (persistent)
+  unsigned long long nhuge;         // windows of the huge class (first in the sorted order)
+  unsigned long long nlarge;        // windows of the huge and large classes
   unsigned long long next;    // next unreserved output slot
   unsigned long long hits;    // exact pair count
   unsigned long long nholes;  // unused chunk ends recorded
@@ -474,6 +481,8 @@ struct PersistParams {
   int stack_cap;
   int stage_n;  // nodes staged in shared memory (multiple of 4), 0 = none
   int parts;    // warps sharing one window (shares of the root's children)
+  bool classes;  // the windows are sorted by class: huge, large, small
+  int split_height;  // nodes of this height are dealt out among a huge window's warps
   int chunk;
   int32_t* fid;
   int32_t* tid;
@@ -498,6 +507,22 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
           smem_addr(dst)),
       "l"(src), "r"(bytes), "r"(bar)
       : "memory");
+}
+
+// Warps sharing a huge window, each walking the levels above the split height
+// and then its own share of the nodes of that height.  A window of side 0.1 on
+// 10M boxes keeps one warp busy for 1.2 ms, so a batch with few such windows
+// waits for the slowest; many of them fill the GPU by themselves, and then the
+// levels walked twice only cost.  Traversal of mixed batches (sides 1e-5 ..
+// 0.1, 10M boxes, 16 warps per CTA) with 1, 2, 4 and 8 warps per huge window:
+//     5k windows (0.1 per warp)  1243    -   411   315 us
+//    60k         (1.5)           1649    -  1189  1216
+//   250k         (6)             4050  3745  3805  4168
+//     1M         (24)           13240 13350 14100     -
+// Road geometry (20k windows, a tenth covering over 1%): 3490 -> 1215 us.
+__device__ __forceinline__ int split_parts_for(long long nhuge, long long warps)
+{
+  return 2 * nhuge < warps ? 8 : nhuge < 2 * warps ? 4 : nhuge < 12 * warps ? 2 : 1;
 }
 
 // kShare: range sharing (the job queue).  Its code needs registers the
@@ -573,7 +598,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
   const long long nq = (long long)P.ctr->nq;
   const int parts = P.parts;
-  const long long ntickets = nq * parts;  // one ticket per (window, share)
+  // one ticket per (window, share); the small windows are small_windows_kernel's
+  const long long nhuge = P.classes ? (long long)P.ctr->nhuge : 0;
+  const int split_parts = split_parts_for(nhuge, (long long)gridDim.x * warps);
+  const long long nsplit = nhuge * split_parts;
+  const long long ntickets = nsplit + ((P.classes ? (long long)P.ctr->nlarge : nq) - nhuge) * parts;
   ChunkEmit emit;
   emit.fid = P.fid;
   emit.tid = P.tid;
@@ -582,7 +611,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   emit.chunk = P.chunk;
   emit.jobs = kShare ? P.jobs : nullptr;
   JobQueue* Q = kShare ? P.jobs : nullptr;
-  (void)warps;
   // a warp counts as active from before its first ticket until it has left
   // the ticket loop, so a waiting warp that sees the tickets gone and no
   // warp active knows no window can publish any more
@@ -595,13 +623,28 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     if (lane_id() == 0) t = atomicAdd(&P.ctr->ticket, 1ull);
     t = __shfl_sync(0xffffffffu, t, 0);
     if ((long long)t >= ntickets) break;
-    const long long qi = parts == 1 ? (long long)t : (long long)t / parts;
-    const int part = parts == 1 ? 0 : (int)((long long)t - qi * parts);
+    long long qi = (long long)t;
+    int part = 0, nparts = 1;
+    Split split;
+    if ((long long)t < nsplit) {
+      qi = (long long)t / split_parts;
+      split.height = P.split_height;
+      split.mask = split_parts - 1;
+      split.part = (int)t & (split_parts - 1);
+    } else {
+      qi -= nsplit;
+      if (parts > 1) {
+        nparts = parts;
+        part = (int)(qi % parts);
+        qi /= parts;
+      }
+      qi += nhuge;
+    }
     int q = order ? (int)order[qi] : (int)qi;
     if (q < 0 || (long long)q >= nq) q = (int)qi;  // only after a sort error (reported)
     emit.begin(q);
     traverse(P.T, C, P.K, lg, lc, P.W.xmin[q], P.W.ymin[q], P.W.xmax[q], P.W.ymax[q], stack,
-             P.stack_cap, emit, &P.ctr->error, part, parts);
+             P.stack_cap, emit, &P.ctr->error, part, nparts, split);
   }
   if (Q) {
     __syncwarp();
@@ -640,6 +683,314 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       }
     }
   }
+}
+
+// ---------------------------------------------------------------------------
+// Small windows (persistent form, windows sorted)
+// ---------------------------------------------------------------------------
+// A window that meets a handful of boxes walks some 20 frontier entries to
+// find them, most of them on the upper levels and the same for its
+// neighbours; one window per warp spent 1600 warp instructions on each (10M
+// boxes, fanout 10, sides up to 1e-3: 1.80 ms per 1M windows, 77% of the
+// issue slots).  Here a warp takes up to 32 windows that are neighbours in
+// Morton order (the same batch: 0.67 ms) and
+//   1. descends once with their bounding box, level by level, while the nodes
+//      it meets fit the frontier (kFrontier): that frontier holds every node
+//      of its level that any of the windows meets;
+//   2. tests every window (one per lane) against the frontier's MBRs;
+//   3. takes the (window, node) pairs K at a time: leaf-parents' boxes are
+//      tested at once, other nodes go on through traverse_group's stack.
+// Only for packed trees over ordinary boxes: a node excluded by the bounding
+// box is excluded by each window, and (NaN aside) a child that a window meets
+// lies under nodes that it meets, so skipping those tests changes nothing.  A
+// NaN in a window opens that side of the bounding box.  Hits are staged in
+// shared memory and flushed densely, one reservation per flush, so nothing is
+// left for the compaction pass.
+constexpr int kSmallWarps = 8;
+constexpr int kFrontier = 96;     // nodes (64: 770, 96: 674, 128: 705 us for the batch above)
+constexpr int kSmallStage = 128;  // staged pairs per warp
+constexpr int kSmallSets = 2;     // pairs tested per step, in multiples of K
+constexpr int kPairChunk = 32;  // frontier nodes whose pairs are listed at a time
+
+struct StageEmit {
+  int2* s_out;  // this warp's staging, kSmallStage pairs
+  int n = 0;
+  int32_t* fid;
+  int32_t* tid;
+  long long cap;
+  unsigned long long* next;
+  long long total = 0;
+  __device__ __forceinline__ long long reserve(long long count)
+  {
+    unsigned long long b = 0;
+    if (lane_id() == 0) b = atomicAdd(next, (unsigned long long)count);
+    total += count;
+    return (long long)__shfl_sync(0xffffffffu, b, 0);
+  }
+  __device__ __forceinline__ void flush()
+  {
+    __syncwarp();
+    if (n > 0) {
+      const long long b = reserve(n);
+      for (int i = (int)lane_id(); i < n; i += 32) {
+        const int2 v = s_out[i];
+        put_pair(fid, tid, b + i, cap, v.x, v.y);
+      }
+      n = 0;
+    }
+    __syncwarp();
+  }
+  // The lanes of mask m (hit) emit (id, window q).
+  __device__ __forceinline__ void hits(uint32_t m, bool hit, int id, int q)
+  {
+    const int c = __popc(m);
+    if (n + c > kSmallStage) flush();
+    if (hit) s_out[n + __popc(m & lanemask_lt())] = make_int2(id, q);
+    n += c;
+  }
+  // Every lane's slot range, 32 ids per warp pass (as emit_small_ranges), each
+  // with its range's window.
+  __device__ __forceinline__ void small_ranges(const int* __restrict__ bid, bool mine, long long first,
+                                               int count, int q)
+  {
+    const int lane = (int)lane_id();
+    const int c = mine ? count : 0;
+    int x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const int all = __shfl_sync(0xffffffffu, x, 31);
+    const int base = (int)first - (x - c);  // sorted slots are below 2^31
+    for (int t0 = 0; t0 < all; t0 += 32) {
+      const int t = t0 + lane;
+      int j = 0;  // lanes whose inclusive prefix is <= t: the owner of t
+#pragma unroll
+      for (int s = 16; s > 0; s >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, x, j + s - 1);
+        if (v <= t) j += s;
+      }
+      const int b = __shfl_sync(0xffffffffu, base, j);
+      const int w = __shfl_sync(0xffffffffu, q, j);
+      const bool ok = t < all;
+      hits(__ballot_sync(0xffffffffu, ok), ok, ok ? __ldg(bid + b + t) : 0, w);
+    }
+  }
+  __device__ __forceinline__ void big_ranges(const int* bid, bool mine, long long first, long long count,
+                                             int q)
+  {
+    uint32_t im = __ballot_sync(0xffffffffu, mine);
+    while (im) {
+      const int src = __ffs(im) - 1;
+      im &= im - 1;
+      const long long c = __shfl_sync(0xffffffffu, count, src);
+      copy_range(bid, __shfl_sync(0xffffffffu, first, src), c, fid, tid, reserve(c), cap,
+                 __shfl_sync(0xffffffffu, q, src));
+    }
+  }
+};
+
+// Shared memory of one warp.  The pair list and the stack follow each other;
+// both are free while the frontier is expanded, which uses their room for the
+// next level's nodes.
+struct SmallSmem {
+  static constexpr size_t kWin = 0;                                     // float4 x 32
+  static constexpr size_t kQ = kWin + 16 * kGroupWindows;               // int x 32
+  static constexpr size_t kMbr = kQ + 4 * kGroupWindows;                // float4 x kFrontier
+  static constexpr size_t kLink = kMbr + 16 * kFrontier;                // int2 x kFrontier
+  static constexpr size_t kOut = kLink + 8 * kFrontier;                 // int2 x kSmallStage
+  static constexpr size_t kPairs = kOut + 8 * kSmallStage;              // uint16 x pairs
+  static constexpr size_t kStack = kPairs + 2 * kGroupWindows * kPairChunk;
+  static_assert(kMbr % 16 == 0 && kPairs % 16 == 0 && kStack % 16 == 0, "16-byte parts");
+  static size_t bytes(int stack_cap)
+  {
+    const size_t a = kStack + sizeof(FrontierEntry) * (size_t)stack_cap;
+    const size_t b = kPairs + 24 * (size_t)kFrontier;
+    return ((a > b ? a : b) + 15) / 16 * 16;
+  }
+};
+
+__global__ void __launch_bounds__(kSmallWarps * 32, 3)
+    small_windows_kernel(PersistParams P, int warp_bytes)
+{
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int lane = (int)lane_id(), warp = threadIdx.x >> 5;
+  unsigned char* my = smem_raw + (size_t)warp * warp_bytes;
+  float4* s_win = (float4*)(my + SmallSmem::kWin);
+  int* s_q = (int*)(my + SmallSmem::kQ);
+  float4* f_mbr = (float4*)(my + SmallSmem::kMbr);
+  int2* f_link = (int2*)(my + SmallSmem::kLink);  // {first child, children}
+  uint16_t* s_pair = (uint16_t*)(my + SmallSmem::kPairs);
+  FrontierEntry* stack = (FrontierEntry*)(my + SmallSmem::kStack);
+  float4* g_mbr = (float4*)(my + SmallSmem::kPairs);  // the next level, while expanding
+  int2* g_link = (int2*)(my + SmallSmem::kPairs + 16 * kFrontier);
+  const TreeView& T = P.T;
+  const int K = P.K;
+  const uint32_t lt = lanemask_lt();
+  int lg, lc;
+  lane_map(T.fanout, lg, lc);
+  const int na = P.sort_ctrl->n_active;
+  const uint32_t* order = na == 0 ? nullptr : ((na & 1) ? P.order1 : P.order0);
+  const long long nlarge = (long long)P.ctr->nlarge, nq = (long long)P.ctr->nq;
+  const long long nsmall = nq - nlarge;
+  // batches shrink towards the end (guided self-scheduling, Polychronopoulos
+  // and Kuck, 1987)
+  const long long share = (long long)gridDim.x * kSmallWarps * 2;
+  StageEmit emit;
+  emit.s_out = (int2*)(my + SmallSmem::kOut);
+  emit.fid = P.fid;
+  emit.tid = P.tid;
+  emit.cap = P.cap;
+  emit.next = &P.ctr->next;
+  unsigned long long t = 0;
+  while (true) {
+    const int want = (int)max(1ll, min((long long)kGroupWindows, (nsmall - (long long)t) / share));
+    if (lane == 0) t = atomicAdd(&P.ctr->small_ticket, (unsigned long long)want);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if ((long long)t >= nsmall) break;
+    const int nw = (int)min((long long)want, nsmall - (long long)t);
+    // the windows, and their bounding box (a NaN opens its side)
+    const float inf = __int_as_float(0x7f800000);
+    float4 w = make_float4(inf, inf, -inf, -inf);
+    if (lane < nw) {
+      const long long qi = nlarge + (long long)t + lane;
+      int q = order ? (int)order[qi] : (int)qi;
+      if (q < 0 || (long long)q >= nq) q = (int)qi;  // only after a sort error (reported)
+      w = make_float4(P.W.xmin[q], P.W.ymin[q], P.W.xmax[q], P.W.ymax[q]);
+      s_q[lane] = q;
+    }
+    s_win[lane] = w;
+    float4 box = make_float4(isnan(w.x) ? -inf : w.x, isnan(w.y) ? -inf : w.y,
+                             isnan(w.z) ? inf : w.z, isnan(w.w) ? inf : w.w);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      box.x = fminf(box.x, __shfl_xor_sync(0xffffffffu, box.x, o));
+      box.y = fminf(box.y, __shfl_xor_sync(0xffffffffu, box.y, o));
+      box.z = fmaxf(box.z, __shfl_xor_sync(0xffffffffu, box.z, o));
+      box.w = fmaxf(box.w, __shfl_xor_sync(0xffffffffu, box.w, o));
+    }
+    // 1. the frontier: from the root (never tested), level by level
+    if (lane == 0) f_link[0] = make_int2(__ldg(T.npos), __ldg(T.nlen));
+    __syncwarp();
+    int nf = 1;
+    int height = T.nlev - 1;  // of the frontier's nodes (0: leaf-parents)
+    while (height > 0) {
+      int ng = 0;
+      for (int e0 = 0; e0 < nf && ng <= kFrontier; e0 += K) {
+        const int e = e0 + lg;
+        bool ok = lg < K && e < nf;
+        const int2 link = f_link[ok ? e : 0];
+        const int i = link.x + lc;
+        ok = ok && lc < link.y && i < T.rsz;
+        float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+        int2 l = make_int2(0, 0);
+        if (ok) {
+          m = make_float4(__ldg(T.nxmin + i), __ldg(T.nymin + i), __ldg(T.nxmax + i), __ldg(T.nymax + i));
+          l = make_int2(__ldg(T.npos + i), __ldg(T.nlen + i));
+        }
+        const bool hit = ok && intersects(box.x, box.y, box.z, box.w, m.x, m.y, m.z, m.w);
+        const uint32_t hm = __ballot_sync(0xffffffffu, hit);
+        const int at = ng + __popc(hm & lt);
+        if (hit && at < kFrontier) {
+          g_mbr[at] = m;
+          g_link[at] = l;
+        }
+        ng += __popc(hm);
+      }
+      __syncwarp();
+      if (ng > kFrontier) break;  // the level does not fit: stay above it
+      for (int i = lane; i < ng; i += 32) {
+        f_mbr[i] = g_mbr[i];
+        f_link[i] = g_link[i];
+      }
+      __syncwarp();
+      nf = ng;
+      height--;
+      if (nf == 0) break;
+    }
+    // 2./3. pairs of windows and frontier nodes, kPairChunk nodes at a time
+    const bool top = height == T.nlev - 1;  // the root itself: never tested
+    for (int c0 = 0; c0 < nf; c0 += kPairChunk) {
+      const int nc = min(kPairChunk, nf - c0);
+      uint32_t mine = 0;
+      if (lane < nw) {
+        if (top) {
+          mine = 1u;
+        } else {
+          for (int i = 0; i < nc; i++) {
+            const float4 m = f_mbr[c0 + i];
+            if (intersects(w.x, w.y, w.z, w.w, m.x, m.y, m.z, m.w)) mine |= 1u << i;
+          }
+        }
+      }
+      const int cnt = __popc(mine);
+      int x = cnt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      const int np = __shfl_sync(0xffffffffu, x, 31);
+      for (int at = x - cnt; mine; mine &= mine - 1)
+        s_pair[at++] = (uint16_t)(lane << 8 | (c0 + __ffs(mine) - 1));
+      __syncwarp();
+      if (height == 0) {
+        // leaf-parents: test their boxes
+        for (int p0 = 0; p0 < np; p0 += kSmallSets * K) {
+          float m1[kSmallSets], n1[kSmallSets], m2[kSmallSets], n2[kSmallSets];
+          int id[kSmallSets], wl[kSmallSets];
+          bool ok[kSmallSets];
+#pragma unroll
+          for (int s = 0; s < kSmallSets; s++) {
+            const int p = p0 + s * K + lg;
+            ok[s] = lg < K && p < np;
+            const uint32_t pr = s_pair[ok[s] ? p : 0];
+            wl[s] = pr >> 8;
+            const int2 link = f_link[pr & 0xFFu];
+            const int j = link.x - T.rsz + lc;
+            ok[s] = ok[s] && lc < link.y && j < T.nbox;
+            m1[s] = n1[s] = m2[s] = n2[s] = 0.f;
+            id[s] = 0;
+            if (ok[s]) {
+              m1[s] = __ldg(T.bxmin + j);
+              n1[s] = __ldg(T.bymin + j);
+              m2[s] = __ldg(T.bxmax + j);
+              n2[s] = __ldg(T.bymax + j);
+              id[s] = __ldg(T.bid + j);
+            }
+          }
+#pragma unroll
+          for (int s = 0; s < kSmallSets; s++) {
+            const float4 v = s_win[wl[s]];
+            const bool hit = ok[s] && intersects(v.x, v.y, v.z, v.w, m1[s], n1[s], m2[s], n2[s]);
+            const uint32_t hm = __ballot_sync(0xffffffffu, hit);
+            if (hm) emit.hits(hm, hit, id[s], s_q[wl[s]]);
+          }
+        }
+      } else {
+        int p = 0;
+        traverse_group<kSmallSets>(
+            T, K, lg, lc, s_win, s_q, stack, P.stack_cap, emit,
+            [&](int sp) {
+              const int m = min(kGroupWindows, np - p);
+              if (m <= 0) return sp;
+              if (lane < m) {
+                const uint32_t pr = s_pair[p + lane];
+                const int2 link = f_link[pr & 0xFFu];
+                stack[sp + lane] = group_entry(link.x, link.y, (int)(pr >> 8), height - 1);
+              }
+              p += m;
+              __syncwarp();
+              return sp + m;
+            },
+            &P.ctr->error);
+      }
+      __syncwarp();
+    }
+  }
+  emit.flush();
+  if (lane == 0 && emit.total) atomicAdd(&P.ctr->hits, (unsigned long long)emit.total);
 }
 
 // Sorts the recorded holes by start: rank by counting (starts are distinct:
@@ -797,16 +1148,43 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Window keys (same Morton key as the boxes) and digit histograms.
-__global__ void window_key_kernel(WindowView W, uint32_t* __restrict__ keys,
-                                  SortCtrl* __restrict__ ctrl)
+// Window keys and digit histograms: the boxes' Morton key, below two class
+// bits when the windows are classed (huge, large, small; the key's two lowest
+// bits make room).  The class is by the boxes a uniform density over the
+// root's MBR gives the window: it only decides which kernel answers it.  The
+// small kernel's lead over one window per warp does not hang on its line (64,
+// 256 and 1024 boxes measured within 4% on mixed batches); the huge line
+// (windows of 4k, 8k, 16k boxes and more split) took 60k mixed windows 1.31,
+// 1.43 and 1.48 ms.  A NaN makes a window large.
+constexpr float kSmallHits = 256.f;
+constexpr float kHugeHits = 4096.f;
+
+__global__ void window_key_kernel(WindowView W, TreeView T, bool classes, QueryCounters* __restrict__ qc,
+                                  uint32_t* __restrict__ keys, SortCtrl* __restrict__ ctrl)
 {
   __shared__ uint32_t sh[kDigits][kBins];
   for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) (&sh[0][0])[i] = 0;
+  classes = classes && T.lvl_odd != nullptr && *T.lvl_odd == 0;
+  float root_w = 0.f, root_h = 0.f;
+  if (classes) {
+    root_w = __ldg(T.nxmax) - __ldg(T.nxmin);
+    root_h = __ldg(T.nymax) - __ldg(T.nymin);
+  }
+  unsigned huge = 0, large = 0;  // large counts both
   __syncthreads();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < W.n;
        i += (long long)gridDim.x * blockDim.x) {
-    uint32_t k = sort_key(W.xmin[i], W.ymin[i], W.xmax[i], W.ymax[i]);
+    const float x1 = W.xmin[i], y1 = W.ymin[i], x2 = W.xmax[i], y2 = W.ymax[i];
+    uint32_t k = sort_key(x1, y1, x2, y2);
+    bool small = false;
+    if (classes) {
+      const float part = fminf(1.f, (x2 - x1) / root_w) * fminf(1.f, (y2 - y1) / root_h);
+      small = part * (float)T.nbox <= kSmallHits && x2 >= x1 && y2 >= y1;
+      const bool big = T.nlev > 1 && !(part * (float)T.nbox <= kHugeHits);
+      k = k >> 2 | (small ? 0xC0000000u : big ? 0u : 0x40000000u);
+      huge += big;
+    }
+    large += !small;
     keys[i] = k;
 #pragma unroll
     for (int d = 0; d < kDigits; d++) atomicAdd(&sh[d][key_digit(k, d)], 1u);
@@ -816,6 +1194,10 @@ __global__ void window_key_kernel(WindowView W, uint32_t* __restrict__ keys,
     uint32_t v = (&sh[0][0])[i];
     if (v) atomicAdd(&ctrl->hist[i], v);
   }
+  large = __reduce_add_sync(0xffffffffu, large);
+  huge = __reduce_add_sync(0xffffffffu, huge);
+  if (large && (threadIdx.x & 31) == 0) atomicAdd(&qc->nlarge, (unsigned long long)large);
+  if (huge && (threadIdx.x & 31) == 0) atomicAdd(&qc->nhuge, (unsigned long long)huge);
   sort_plan(ctrl, W.n, kDigits);
 }
 
@@ -1055,8 +1437,8 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
 // host: `pre` (reset the counters, order the windows), the traversal kernel,
 // and `post` (sort the unused chunk ends, compact, write the result block).
 // A plan records all three as one CUDA graph.
-static void enqueue_pre(const WindowView& W, int64_t max_nq, const PersistScratch& S, bool sort,
-                        cudaStream_t stream)
+static void enqueue_pre(const TreeView& T, const WindowView& W, int64_t max_nq,
+                        const PersistScratch& S, bool sort, bool classes, cudaStream_t stream)
 {
   // counters (keep nq), the job queue's ready flags and the sort's zeroed block
   cudaMemsetAsync(S.ctr, 0, offsetof(QueryCounters, nq), stream);
@@ -1065,7 +1447,8 @@ static void enqueue_pre(const WindowView& W, int64_t max_nq, const PersistScratc
     const int sms = sm_count();
     cudaMemsetAsync(S.sort_zero, 0, sort_zero_bytes(max_nq), stream);
     int g = (int)std::min<int64_t>(cdiv(max_nq, 256), (int64_t)sms * 4);
-    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, S.cols.key[0], sort_ctrl(S.sort_zero));
+    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, T, classes, S.ctr, S.cols.key[0],
+                                                          sort_ctrl(S.sort_zero));
     sort_passes(S.cols, W.n, kDigits, S.sort_zero, stream);
     CRT_LAUNCHED(1);
   }
@@ -1077,7 +1460,19 @@ struct TraverseLaunch {
   int grid;
   int threads;
   const void* fn;
+  // the small windows' launch (P.classes)
+  PersistParams small;
+  int small_grid;
+  int small_warp_bytes;
 };
+
+// Whether the windows are classed: sorted, and a packed tree of fanout <= 32
+// whose boxes were scanned (a box that is not ordinary makes every window
+// large, on the device).
+static bool window_classes(const TreeView& T, bool sort)
+{
+  return sort && T.nlev > 0 && T.lvl_odd != nullptr && T.fanout <= 32 && T.rsz > 0;
+}
 
 static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
                                     const PersistScratch& S, bool sort, int stage_n,
@@ -1097,6 +1492,10 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
   P.stack_cap = sh.stack_cap;
   P.stage_n = ps.stage_n;
   P.parts = parts;
+  P.classes = window_classes(T, sort);
+  P.split_height = 0;  // the first height whose nodes hold 256 boxes, at most the root's children's
+  for (int64_t span = T.fanout; span < 256 && P.split_height < T.nlev - 2; span *= T.fanout)
+    P.split_height++;
   P.chunk = chunk;
   P.fid = fid;
   P.tid = tid;
@@ -1109,6 +1508,20 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
   L.threads = ps.v->threads;
   L.fn = ps.v->fn;
   L.grid = persistent_grid(*ps.v, L.smem);
+  if (P.classes) {
+    L.small = P;
+    // as one window's stack, with kSmallSets sets per step, a refill and the
+    // entries left when it ran
+    const int cap = (levels_of(T.nbox, T.fanout) - 1) * kSmallSets * sh.K * T.fanout + kGroupWindows +
+                    kSmallSets * sh.K;
+    L.small.stack_cap = (cap + 31) / 32 * 32;
+    L.small_warp_bytes = (int)SmallSmem::bytes(L.small.stack_cap);
+    const size_t smem = (size_t)L.small_warp_bytes * kSmallWarps;
+    int per_sm = 0;
+    cudaFuncSetAttribute(small_windows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, small_windows_kernel, kSmallWarps * 32, smem);
+    L.small_grid = std::max(per_sm, 1) * sm_count();
+  }
   return L;
 }
 
@@ -1118,6 +1531,12 @@ static cudaError_t launch_traverse(const TraverseLaunch& L, cudaStream_t stream)
   void* args[] = {(void*)&L.P};
   cudaError_t e = cudaLaunchKernel(L.fn, dim3(L.grid), dim3(L.threads), args, L.smem, stream);
   CRT_LAUNCHED(1);
+  if (e == cudaSuccess && L.P.classes) {
+    small_windows_kernel<<<L.small_grid, kSmallWarps * 32, (size_t)L.small_warp_bytes * kSmallWarps,
+                           stream>>>(L.small, L.small_warp_bytes);
+    CRT_LAUNCHED(1);
+    e = cudaGetLastError();
+  }
   return e;
 }
 
@@ -1263,7 +1682,7 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   attach_levels(T, lt, scr + S.bytes, stream);
   set_nq_kernel<<<1, 1, 0, stream>>>(S.ctr, nq);
   CRT_LAUNCHED(1);
-  enqueue_pre(W, nq, S, sort, stream);
+  enqueue_pre(T, W, nq, S, sort, window_classes(T, sort), stream);
   cudaError_t e = launch_traverse(make_traverse(T, W, S, sort, stage_n, fid, tid, capacity, chunk,
                                                 opts.warps_per_cta, parts),
                                   stream);
@@ -1522,7 +1941,7 @@ int plan_create(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   if (e == cudaSuccess) e = cudaEventCreate(&p->own[1]);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    enqueue_pre(p->W, max_nq, p->S, p->sort, cs);
+    enqueue_pre(p->T, p->W, max_nq, p->S, p->sort, window_classes(p->T, p->sort), cs);
     cudaError_t le = cudaEventRecordWithFlags(p->own[0], cs, cudaEventRecordExternal);
     if (le == cudaSuccess) le = launch_traverse(p->traverse, cs);
     if (le == cudaSuccess) le = cudaEventRecordWithFlags(p->own[1], cs, cudaEventRecordExternal);
@@ -1581,7 +2000,7 @@ int plan_launch(void* hp, cudaStream_t stream)
   if (e != cudaSuccess) return cuda_fail(e, "plan_launch");
   // window keys and four sort passes; the traversal; hole sort,
   // prefix and compaction
-  CRT_LAUNCHED((p->sort ? 5 : 0) + 1 + 3);
+  CRT_LAUNCHED((p->sort ? 5 : 0) + 1 + (p->traverse.P.classes ? 1 : 0) + 3);
   return CRT_OK;
 }
 

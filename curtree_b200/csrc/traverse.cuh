@@ -342,12 +342,21 @@ struct ChildTest {
   bool leaf;  // a box slot (counted as a leaf test)
 };
 
+// A window shared by several warps below the root: every warp walks the nodes
+// above `height`, and a node of that height (or a contained one above it)
+// belongs to the warp `part` that its index names.  mask == 0: not shared.
+struct Split {
+  int height = 0;
+  int mask = 0;  // parts - 1, parts a power of two
+  int part = 0;
+};
+
 // Tests child c of popped entry g (of k popped; lane e of the warp holds
 // entry e): a leaf box against the window, or an inner node (intersects:
 // push its children range; contained: emit its boxes' slot range).
 __device__ __forceinline__ void test_child(const TreeView& T, const NodeCache& C, FrontierEntry e,
                                            int k, int g, int c, bool contain, float x1, float y1,
-                                           float x2, float y2, ChildTest& t)
+                                           float x2, float y2, const Split& split, ChildTest& t)
 {
   const int gs = min(g, k - 1);
   const int pos = __shfl_sync(0xffffffffu, e.x, gs);
@@ -377,7 +386,12 @@ __device__ __forceinline__ void test_child(const TreeView& T, const NodeCache& C
     load_node_box(T, C, child, a, b, cc, d);
     load_node_link(T, C, child, t.cpos, t.clen);
     t.push = intersects(x1, y1, x2, y2, a, b, cc, d);
-    if (contain && t.push && x1 <= a && cc <= x2 && y1 <= b && d <= y2) {
+    const bool inside = contain && t.push && x1 <= a && cc <= x2 && y1 <= b && d <= y2;
+    // another warp's share of the window
+    if (split.mask && (hc == split.height || (inside && hc > split.height)) &&
+        (child & split.mask) != split.part) {
+      t.push = false;
+    } else if (inside) {
       t.inside = true;
       t.push = false;
       const long long span = __ldg(T.lvl_span + hc);
@@ -396,7 +410,8 @@ template <class Emit, bool kContain = true>
 __device__ __forceinline__ void traverse(const TreeView& T, const NodeCache& C, int K,
                                          int lane_g, int lane_c, float x1, float y1, float x2,
                                          float y2, FrontierEntry* stack, int stack_cap,
-                                         Emit& emit, int* err, int part = 0, int nparts = 1)
+                                         Emit& emit, int* err, int part = 0, int nparts = 1,
+                                         Split split = Split())
 {
   const int lane = (int)lane_id();
   const uint32_t lt = lanemask_lt();
@@ -447,8 +462,8 @@ __device__ __forceinline__ void traverse(const TreeView& T, const NodeCache& C, 
     const int span = f <= 32 ? 32 : f;  // children covered per node group
     for (int base = 0; base < span; base += 32) {
       ChildTest t;
-      if (f <= 32) test_child(T, C, e, k, lane_g, lane_c, contain, x1, y1, x2, y2, t);
-      else test_child(T, C, e, k, 0, base + lane, contain, x1, y1, x2, y2, t);
+      if (f <= 32) test_child(T, C, e, k, lane_g, lane_c, contain, x1, y1, x2, y2, split, t);
+      else test_child(T, C, e, k, 0, base + lane, contain, x1, y1, x2, y2, split, t);
       if constexpr (Emit::kCountsTests) emit.leaf_tests(__popc(__ballot_sync(0xffffffffu, t.leaf)));
       const uint32_t pm = __ballot_sync(0xffffffffu, t.push);
       if (pm) {
@@ -467,6 +482,106 @@ __device__ __forceinline__ void traverse(const TreeView& T, const NodeCache& C, 
         if (__any_sync(0xffffffffu, small)) emit.small_ranges(T.bid, small, t.rfirst, (int)t.rcount);
         const bool big = t.inside && !small;
         if (__any_sync(0xffffffffu, big)) emit.big_ranges(T.bid, big, t.rfirst, t.rcount);
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Warp traversal of several windows at once (fanout <= 32)
+// ---------------------------------------------------------------------------
+// The warp's stack holds entries of up to 32 windows (each entry names its
+// window); a step pops kSets * K entries of any of them, and the loads of all
+// their children are in flight together.  An entry's `y` is: children count
+// (bits 0-7), window (bits 8-12), height of the nodes in the range (bits
+// 24-31).  refill(sp) may push entries when a step would not be full (sp <
+// kSets * K) and returns the new stack size; below its entries the stack keeps
+// the depth order of one window's, so it never holds more than kSets * K *
+// fanout entries per level, plus the refill's kGroupWindows and the kSets * K
+// left when it ran.  Only for packed trees over ordinary boxes.
+constexpr int kGroupWindows = 32;
+constexpr int kGroupLenMask = 0xFF;
+
+__device__ __forceinline__ FrontierEntry group_entry(int pos, int len, int window, int height)
+{
+  // at most 32 children are looked at (lane_c < fanout)
+  return make_int2(pos, min(max(len, 0), 32) | window << 8 | height << 24);
+}
+
+template <int kSets, class Emit, class Refill>
+__device__ __forceinline__ void traverse_group(const TreeView& T, int K, int lane_g, int lane_c,
+                                               const float4* s_win, const int* s_q,
+                                               FrontierEntry* stack, int stack_cap, Emit& emit,
+                                               Refill refill, int* err)
+{
+  const uint32_t lt = lanemask_lt();
+  int sp = 0;
+  while (true) {
+    if (sp < kSets * K) sp = refill(sp);
+    if (sp == 0) return;
+    const int k = min(sp, kSets * K);
+    sp -= k;
+    // popped entries stack[sp .. sp+k): lower index = shallower.  Every set's
+    // loads are issued before the first test; boxes and nodes share them, so
+    // a step that meets both waits one round trip.
+    float m1[kSets], n1[kSets], m2[kSets], n2[kSets];
+    int ref[kSets], len[kSets], child[kSets], ey[kSets];
+    bool ok[kSets], leaf[kSets];
+#pragma unroll
+    for (int s = 0; s < kSets; s++) {
+      const int at = s * K + lane_g;
+      ok[s] = lane_g < K && at < k;
+      const FrontierEntry e = stack[sp + (ok[s] ? at : 0)];
+      ey[s] = e.y;
+      child[s] = e.x + lane_c;
+      leaf[s] = e.x >= T.rsz;
+      const int j = leaf[s] ? child[s] - T.rsz : child[s];
+      ok[s] = ok[s] && lane_c < (e.y & kGroupLenMask) && j < (leaf[s] ? T.nbox : T.rsz);
+      m1[s] = n1[s] = m2[s] = n2[s] = 0.f;
+      ref[s] = len[s] = 0;
+      if (ok[s]) {
+        m1[s] = __ldg((leaf[s] ? T.bxmin : T.nxmin) + j);
+        n1[s] = __ldg((leaf[s] ? T.bymin : T.nymin) + j);
+        m2[s] = __ldg((leaf[s] ? T.bxmax : T.nxmax) + j);
+        n2[s] = __ldg((leaf[s] ? T.bymax : T.nymax) + j);
+        ref[s] = __ldg((leaf[s] ? T.bid : T.npos) + j);  // a box's id, a node's first child
+        if (!leaf[s]) len[s] = __ldg(T.nlen + j);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int s = 0; s < kSets; s++) {
+      const int wl = (ey[s] >> 8) & (kGroupWindows - 1);
+      const float4 w = s_win[wl];
+      const bool meets = ok[s] && intersects(w.x, w.y, w.z, w.w, m1[s], n1[s], m2[s], n2[s]);
+      const bool inside = meets && !leaf[s] && w.x <= m1[s] && m2[s] <= w.z && w.y <= n1[s] && n2[s] <= w.w;
+      const bool push = meets && !leaf[s] && !inside;
+      const int h = (int)((uint32_t)ey[s] >> 24);
+      const uint32_t pm = __ballot_sync(0xffffffffu, push);
+      if (pm) {
+        const int np = __popc(pm);
+        if (sp + np > stack_cap) {
+          // cannot happen with the host-sized stack; never write past it
+          raise_error(err, CRT_ERR_NOT_SUPPORTED);
+          return;
+        }
+        if (push) stack[sp + __popc(pm & lt)] = group_entry(ref[s], len[s], wl, max(h - 1, 0));
+        sp += np;
+      }
+      const uint32_t hm = __ballot_sync(0xffffffffu, meets && leaf[s]);
+      if (hm) emit.hits(hm, meets && leaf[s], ref[s], s_q[wl]);
+      if (__any_sync(0xffffffffu, inside)) {
+        long long first = 0, count = 0;
+        if (inside) {
+          const long long span = __ldg(T.lvl_span + h);
+          first = (long long)(child[s] - __ldg(T.lvl_first + h)) * span;
+          count = min((long long)T.nbox - first, span);
+        }
+        const bool small = inside && count < kSmallRange;
+        if (__any_sync(0xffffffffu, small)) emit.small_ranges(T.bid, small, first, (int)count, s_q[wl]);
+        const bool big = inside && !small;
+        if (__any_sync(0xffffffffu, big)) emit.big_ranges(T.bid, big, first, count, s_q[wl]);
       }
     }
     __syncwarp();
