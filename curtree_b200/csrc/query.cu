@@ -23,7 +23,7 @@
 //               in Morton order of the window centres (neighbouring windows
 //               share tree paths, so the tree stays in L2); the top tree levels
 //               are staged in shared memory with bulk async copies; hits go to
-//               4096-slot chunks a warp reserves with one atomic, and a
+//               chunks a warp reserves with one atomic, and a
 //               compaction pass moves the tail of the array into the unused
 //               ends of each warp's last chunk so the output is dense.
 //               On sorted windows over packed trees the windows are classed by
@@ -993,75 +993,78 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 3)
   if (lane == 0 && emit.total) atomicAdd(&P.ctr->hits, (unsigned long long)emit.total);
 }
 
-// Sorts the recorded holes by start: rank by counting (starts are distinct:
-// holes do not overlap), one hole per thread, all starts streamed through
-// shared memory in tiles.
-constexpr int kHoleTile = 2048;
+// Sorts the recorded holes by start and makes the exclusive prefix of their
+// lengths: a hole's rank is the number of holes before it (starts are
+// distinct: holes do not overlap) and its prefix their total length.  A CTA
+// takes kRankHoles holes, one per lane, and deals all holes out among its
+// warps, which read each from shared memory once for 32 comparisons.  Bound by
+// the issue of n^2 / 32 comparisons: 28 us for 7104 holes; one thread per hole
+// with a serial loop, and a prefix pass of its own, took 94 us.
+constexpr int kRankHoles = 32;
+constexpr int kRankWarps = 8;
+constexpr int kRankTile = 1024;
 
-__global__ void __launch_bounds__(256)
-    hole_sort_kernel(const Hole* __restrict__ holes, Hole* __restrict__ sorted,
-                     const QueryCounters* __restrict__ ctr, long long max_holes)
+__global__ void __launch_bounds__(kRankWarps * 32)
+    hole_rank_kernel(const Hole* __restrict__ holes, Hole* __restrict__ sorted,
+                     long long* __restrict__ cum, const QueryCounters* __restrict__ ctr,
+                     long long max_holes)
 {
-  __shared__ long long s_start[kHoleTile];
-  const long long nh = min((long long)ctr->nholes, max_holes);
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if ((long long)blockIdx.x * blockDim.x >= nh) return;  // whole CTA idle
-  const long long my = i < nh ? holes[i].start : 0;
-  long long r = 0;
-  for (long long t0 = 0; t0 < nh; t0 += kHoleTile) {
-    const int m = (int)min((long long)kHoleTile, nh - t0);
-    __syncthreads();
-    for (int k = threadIdx.x; k < m; k += blockDim.x) s_start[k] = holes[t0 + k].start;
-    __syncthreads();
-    for (int k = 0; k < m; k++) r += s_start[k] < my;
+  __shared__ __align__(16) Hole s_hole[kRankTile];
+  __shared__ int s_rank[kRankHoles];
+  __shared__ unsigned long long s_before[kRankHoles];
+  const int nh = (int)min((long long)ctr->nholes, max_holes);
+  const int lane = (int)lane_id(), warp = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * kRankHoles;
+  if (i0 >= nh) {  // whole CTA idle
+    if (nh == 0 && blockIdx.x == 0 && threadIdx.x == 0) cum[0] = 0;
+    return;
   }
-  if (i < nh) sorted[r] = holes[i];
+  if (threadIdx.x < kRankHoles) {
+    s_rank[threadIdx.x] = 0;
+    s_before[threadIdx.x] = 0;
+  }
+  const Hole my = holes[min(i0 + lane, nh - 1)];
+  int r = 0;
+  unsigned long long before = 0;
+  for (int t0 = 0; t0 < nh; t0 += kRankTile) {
+    const int m = min(kRankTile, nh - t0);
+    __syncthreads();
+    for (int k = threadIdx.x; k < m; k += blockDim.x) s_hole[k] = holes[t0 + k];
+    __syncthreads();
+    const int k1 = min(m, (warp + 1) * (kRankTile / kRankWarps));
+    for (int k = warp * (kRankTile / kRankWarps); k < k1; k++) {
+      const Hole h = s_hole[k];
+      if (h.start < my.start) {
+        r++;
+        before += (unsigned long long)h.len;
+      }
+    }
+  }
+  __syncthreads();
+  atomicAdd(&s_rank[lane], r);
+  atomicAdd(&s_before[lane], before);
+  __syncthreads();
+  if (threadIdx.x < kRankHoles && i0 + lane < nh) {
+    const int rank = s_rank[lane];
+    sorted[rank] = my;
+    cum[rank] = (long long)s_before[lane];
+    if (rank == nh - 1) cum[nh] = (long long)s_before[lane] + my.len;
+  }
 }
 
-// Exclusive prefix of the sorted hole lengths (one CTA).
-__global__ void __launch_bounds__(kScanThreads)
-    hole_prefix_kernel(const Hole* __restrict__ sorted, long long* __restrict__ cum,
-                       const QueryCounters* __restrict__ ctr, long long max_holes)
+// First index of [0, n) at which `pred` (true, then false) is false, n if
+// none: the CTA tests one pivot per thread and round, two rounds for 2^16
+// indices, instead of a chain of log2 n dependent loads.  Every thread calls.
+template <class Pred>
+__device__ __forceinline__ int block_partition(int n, Pred pred)
 {
-  __shared__ long long s_warp[32];
-  __shared__ long long s_tot;
-  const long long nh = min((long long)ctr->nholes, max_holes);
-  long long carry = 0;
-  for (long long b0 = 0; b0 < nh; b0 += kScanThreads) {
-    long long i = b0 + threadIdx.x;
-    long long v = i < nh ? sorted[i].len : 0;
-    long long x = block_incl_scan(v, s_warp);
-    if (i < nh) cum[i] = carry + x - v;
-    if (threadIdx.x == kScanThreads - 1) s_tot = x;
-    __syncthreads();
-    carry += s_tot;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) cum[nh] = carry;
-}
-
-// Hole slots in [0, x): cum[i] + min(x - st[i], len[i]) for the last hole
-// starting before x.
-__device__ __forceinline__ long long holes_below(const Hole* h, const long long* cum, long long nh,
-                                                 long long x)
-{
-  long long lo = 0, hi = nh;  // first hole with start >= x
-  while (lo < hi) {
-    long long m = (lo + hi) >> 1;
-    if (h[m].start < x) lo = m + 1; else hi = m;
-  }
-  if (lo == 0) return 0;
-  const long long i = lo - 1;
-  return cum[i] + min(x - h[i].start, h[i].len);
-}
-
-// First hole (sorted by start) whose start is >= x.
-__device__ __forceinline__ long long hole_at_or_after(const Hole* h, long long nh, long long x)
-{
-  long long lo = 0, hi = nh;
-  while (lo < hi) {
-    long long m = (lo + hi) >> 1;
-    if (h[m].start < x) lo = m + 1; else hi = m;
+  int lo = 0, end = n;
+  while (lo < end) {
+    const int step = (end - lo + (int)blockDim.x - 1) / (int)blockDim.x;
+    const int i = lo + ((int)threadIdx.x + 1) * step - 1;
+    const int c = __syncthreads_count(i < end && pred(i));
+    end = min(end, lo + (c + 1) * step - 1);
+    lo += c * step;
   }
   return lo;
 }
@@ -1070,17 +1073,19 @@ __device__ __forceinline__ long long hole_at_or_after(const Hole* h, long long n
 // the output is dense [0, T); then writes the result block.  The B pairs to
 // move are the data slots of [T, next) in order, and their destinations the
 // hole slots below T in order: both are runs, so each CTA takes a piece of
-// kMovePiece consecutive moves, finds where its sources and destinations
-// start with binary searches, and then copies run by run with coalesced
-// accesses.
-constexpr long long kMovePiece = 8192;
+// kMovePiece consecutive moves, finds the hole it starts to fill and the data
+// it starts from, and then copies run by run with coalesced accesses.  Bound
+// by the latency of a piece's searches and runs, so pieces are short: 3.6M
+// moves over 7104 holes take 37 us; with binary searches nested in one another
+// and pieces of 8192 they took 96 us.
+constexpr int kMovePiece = 2048;
 
 __global__ void __launch_bounds__(256)
     compact_kernel(const Hole* __restrict__ h, const long long* __restrict__ cum,
                    QueryCounters* __restrict__ ctr, long long max_holes, int32_t* fid,
                    int32_t* tid, long long cap, crt_query_result* __restrict__ res)
 {
-  const long long nh = min((long long)ctr->nholes, max_holes);
+  const int nh = (int)min((long long)ctr->nholes, max_holes);
   const long long T = (long long)ctr->hits;
   const long long R = (long long)ctr->next;
   const bool overflow = R > cap;
@@ -1091,33 +1096,24 @@ __global__ void __launch_bounds__(256)
     res->error = ctr->error;
   }
   if (overflow || ctr->error || nh == 0) return;
-  const long long B = holes_below(h, cum, nh, T);  // pairs to move
+  // holes [0, above) start below T; B hole slots lie below T
+  const int above = block_partition(nh, [&](int i) { return h[i].start < T; });
+  long long B = 0;
+  if (above > 0) B = cum[above - 1] + min(T - h[above - 1].start, h[above - 1].len);
   for (long long r0 = (long long)blockIdx.x * kMovePiece; r0 < B;
        r0 += (long long)gridDim.x * kMovePiece) {
-    long long rem = min(kMovePiece, B - r0);
-    // destination of move r0: the r0-th hole slot below T
-    long long a = 0;
-    {
-      long long lo = 0, hi = nh;  // last hole with cum <= r0
-      while (hi - lo > 1) {
-        const long long m = (lo + hi) >> 1;
-        if (cum[m] <= r0) lo = m; else hi = m;
-      }
-      a = lo;
-    }
+    long long rem = min((long long)kMovePiece, B - r0);
+    // destination of move r0: the r0-th hole slot, in the last hole with at
+    // most r0 hole slots before it
+    int a = block_partition(above, [&](int i) { return cum[i] <= r0; }) - 1;
+    if (a < 0) a = 0;
     long long d = h[a].start + (r0 - cum[a]);
-    // source of move r0: the smallest x >= T with r0 + 1 data slots in [T, x]
-    long long s = T;
-    {
-      long long lo = T, hi = R - 1;
-      while (lo < hi) {
-        const long long m = (lo + hi) >> 1;
-        const long long data = (m + 1 - T) - (holes_below(h, cum, nh, m + 1) - B);
-        if (data >= r0 + 1) hi = m; else lo = m + 1;
-      }
-      s = lo;
-    }
-    long long jn = hole_at_or_after(h, nh, s + 1);  // next hole above the source
+    // source of move r0: hole `above + i` has (start - T) - (cum - B) data
+    // slots of [T, ...) before it; the r0-th lies past those with at most r0
+    int jn = above + block_partition(nh - above, [&](int i) {
+      return h[above + i].start - T - (cum[above + i] - B) <= r0;
+    });  // next hole above the source
+    long long s = T + r0 + (cum[jn] - B);
     while (rem > 0) {
       const long long src_end = jn < nh ? h[jn].start : R;
       const long long dst_end = min(h[a].start + h[a].len, T);
@@ -1322,7 +1318,12 @@ static TraversalShape traversal_shape(int64_t nbox, int fanout)
   return s;
 }
 
-constexpr int kDefaultChunk = 4096;
+// Chunk of a query that names none; the capacity it asks for (query_capacity)
+// leaves room for 4096-slot chunks.  A chunk's unused end is moved by the
+// compaction: 213M pairs of a road batch leave 72 us of moves at 1024 slots,
+// 145 at 4096, with the same traversal time.
+constexpr int kDefaultChunk = 1024;
+constexpr int kDefaultChunkRoom = 4096;
 
 // Persistent traversal variants: CTA width and CTAs per SM, which fix the
 // register budget (65536 / (threads x CTAs)).  Wider CTAs share one staged
@@ -1381,7 +1382,7 @@ static PersistShape persist_shape(int stack_cap, int stage_n, int warps_per_cta)
 int64_t query_capacity(int64_t pairs, const crt_query_opts& o)
 {
   if (o.mode == CRT_QUERY_PLAIN) return pairs;
-  const int chunk = o.chunk > 0 ? o.chunk : kDefaultChunk;
+  const int chunk = o.chunk > 0 ? o.chunk : kDefaultChunkRoom;
   // every resident warp may leave one partly used chunk
   const int64_t warps = (int64_t)sm_count() * 64;  // resident warps per SM at most
   return pairs + warps * chunk;
@@ -1544,12 +1545,11 @@ static void enqueue_post(const PersistScratch& S, int32_t* fid, int32_t* tid, lo
                          crt_query_result* res, cudaStream_t stream)
 {
   const int sms = sm_count();
-  hole_sort_kernel<<<std::max(1, (int)cdiv(S.max_holes, 256)), 256, 0, stream>>>(
-      S.holes, S.sorted, S.ctr, S.max_holes);
-  hole_prefix_kernel<<<1, kScanThreads, 0, stream>>>(S.sorted, S.cum, S.ctr, S.max_holes);
-  compact_kernel<<<sms * 4, 256, 0, stream>>>(S.sorted, S.cum, S.ctr, S.max_holes, fid, tid,
+  hole_rank_kernel<<<std::max(1, (int)cdiv(S.max_holes, kRankHoles)), kRankWarps * 32, 0, stream>>>(
+      S.holes, S.sorted, S.cum, S.ctr, S.max_holes);
+  compact_kernel<<<sms * 8, 256, 0, stream>>>(S.sorted, S.cum, S.ctr, S.max_holes, fid, tid,
                                               cap, res);
-  CRT_LAUNCHED(3);
+  CRT_LAUNCHED(2);
 }
 
 // Nodes of the root and the `levels` whole tree levels below it, rounded up
@@ -1998,9 +1998,9 @@ int plan_launch(void* hp, cudaStream_t stream)
     e = cudaGraphLaunch(p->exec, stream);
   }
   if (e != cudaSuccess) return cuda_fail(e, "plan_launch");
-  // window keys and four sort passes; the traversal; hole sort,
-  // prefix and compaction
-  CRT_LAUNCHED((p->sort ? 5 : 0) + 1 + (p->traverse.P.classes ? 1 : 0) + 3);
+  // window keys and four sort passes; the traversal; hole ranks and
+  // compaction
+  CRT_LAUNCHED((p->sort ? 5 : 0) + 1 + (p->traverse.P.classes ? 1 : 0) + 2);
   return CRT_OK;
 }
 
