@@ -79,15 +79,80 @@ static bool tree_ok(const crt_rtree_f32* t)
 // one's output before its exact count is known.
 static std::atomic<double> g_pairs_per_window{64.0};
 
-// The drop-in query runs into a working buffer from the stream-ordered pool
-// (sized from the last call's pairs per window, re-run once at the exact size
-// if that was too small), then copies the pairs into two exact-size arrays
-// from the same pool, which the caller frees with cudaFree as the reference's
-// idpair_d_free does (src/utility.cuh:164-195).  Batches below
-// kDropinPersistentMin windows take the plain form: its fixed cost (no
-// window sort, no chunk compaction) is far below the persistent form's,
-// which wins on large batches.
+// The drop-in query runs into buffers from the stream-ordered pool (sized from
+// the last call's pairs per window, re-run once at the exact size if that was
+// too small) and returns two arrays from the same pool, which the caller frees
+// with cudaFree as the reference's idpair_d_free does
+// (src/utility.cuh:164-195).  Batches below kDropinPersistentMin windows take
+// the dense form, straight into the two arrays: its fixed cost (no window
+// sort, no compaction) is far below the persistent form's, which wins on large
+// batches.
 constexpr int64_t kDropinPersistentMin = 32768;
+// Slots of a returned array past its pairs that are not worth a copy into an
+// exact one.
+constexpr int64_t kSpareSlots = 65536;
+
+// Small batches.
+static int query_dropin_dense(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
+                              const crt_bbox_f32* d_qbox, crt_idpair* d_dq, cudaStream_t stream)
+{
+  const int64_t nq = d_qbox->sz;
+  int64_t cap = (int64_t)(g_pairs_per_window.load() * (double)nq * 1.25) + 1024;
+  int64_t pairs = 0;
+  int32_t* out[2] = {nullptr, nullptr};
+  auto allocate = [&](int32_t** a, int64_t slots) {
+    for (int c = 0; c < 2; c++)
+      if (cudaMallocAsync((void**)&a[c], sizeof(int32_t) * (size_t)std::max<int64_t>(slots, 1),
+                          stream) != cudaSuccess) {
+        cudaGetLastError();
+        a[c] = nullptr;
+        return fail(CRT_ERR_OOM, "query: output allocation failed");
+      }
+    return (int)CRT_OK;
+  };
+  auto release = [&](int32_t** a) {
+    for (int c = 0; c < 2; c++) {
+      if (a[c]) cudaFreeAsync(a[c], stream);
+      a[c] = nullptr;
+    }
+  };
+  int rc = CRT_OK;
+  for (int attempt = 0; attempt < 2; attempt++) {
+    rc = allocate(out, cap);
+    if (rc == CRT_OK) rc = query_dense(*d_rt, *d_rbox, *d_qbox, out[0], out[1], cap, &pairs, stream);
+    if (rc != CRT_OK || pairs <= cap) break;
+    release(out);
+    if (pairs > INT32_MAX) break;
+    cap = pairs;  // exact: the retry cannot overflow
+  }
+  if (rc == CRT_OK && pairs > INT32_MAX)
+    rc = fail(CRT_ERR_OVERFLOW_INT32, "query: more than INT32_MAX pairs; use crt_query_into_f32");
+  if (rc == CRT_OK && pairs > cap) rc = fail(CRT_ERR_CUDA, "query: output overflow after retry");
+  if (rc == CRT_OK && cap - pairs > std::max(kSpareSlots, pairs)) {
+    int32_t* exact[2] = {nullptr, nullptr};
+    rc = allocate(exact, pairs);
+    cudaError_t e = cudaSuccess;
+    for (int c = 0; c < 2 && rc == CRT_OK && pairs > 0 && e == cudaSuccess; c++)
+      e = cudaMemcpyAsync(exact[c], out[c], sizeof(int32_t) * (size_t)pairs, cudaMemcpyDeviceToDevice,
+                          stream);
+    std::swap(out[0], exact[0]);
+    std::swap(out[1], exact[1]);
+    release(exact);
+    const cudaError_t es = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) e = es;
+    if (rc == CRT_OK && e != cudaSuccess) rc = cuda_fail(e, "query: copy");
+  }
+  if (rc != CRT_OK) {
+    release(out);
+    cudaStreamSynchronize(stream);
+    return rc;
+  }
+  if (nq > 0) g_pairs_per_window.store(std::max(1.0, (double)pairs / (double)nq));
+  d_dq->sz = (int)pairs;
+  d_dq->fid = out[0];
+  d_dq->tid = out[1];
+  return CRT_OK;
+}
 
 static int query_dropin(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
                         const crt_bbox_f32* d_qbox, crt_idpair* d_dq, cudaStream_t stream)
@@ -98,7 +163,12 @@ static int query_dropin(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
   crt_query_opts o;
   crt_query_opts_default(&o);
   const int64_t nq = d_qbox->sz;
-  if (nq < kDropinPersistentMin) o.mode = CRT_QUERY_PLAIN;
+  if (d_rt->sz > 0 && d_rt->fanout < 2) return fail(CRT_ERR_INVALID_ARG, "query: fanout < 2");
+  if (nq < kDropinPersistentMin) {
+    if (query_dense_fits(d_rbox->sz, d_rt->fanout))
+      return query_dropin_dense(d_rt, d_rbox, d_qbox, d_dq, stream);
+    o.mode = CRT_QUERY_PLAIN;
+  }
   int64_t want = (int64_t)(g_pairs_per_window.load() * (double)nq * 1.25) + 1024;
   crt_query_result* res = nullptr;
   if (cudaMallocAsync((void**)&res, sizeof(crt_query_result), stream) != cudaSuccess) {

@@ -29,6 +29,9 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
                int32_t* fid, int32_t* tid, int64_t capacity, crt_query_result* d_result,
                int64_t* d_offsets, const crt_query_opts& opts, cudaStream_t stream);
 int64_t query_capacity(int64_t pairs, const crt_query_opts& opts);
+bool query_dense_fits(int64_t nbox, int fanout);
+int query_dense(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,
+                int32_t* fid, int32_t* tid, int64_t cap, int64_t* pairs, cudaStream_t stream);
 
 // Host parser of the reference's MBR text format (io.cu), with the rules of
 // readMBR's fscanf(fp, "%f,%f,%f,%f,%d,%d,%d\n", ...): one record at p (the

@@ -16,9 +16,11 @@
 // stack ordered by depth, so it never holds more than K*fanout entries per
 // level: (levels - 1) * K * fanout + 1 in total, which the host sizes exactly.
 //
-// Two forms:
+// Three forms:
 //   plain       one warp per window in input order, a count pass, an int64
 //               exclusive scan and a write pass: output grouped by window.
+//   dense       the drop-in query's small batches: one warp (or several) per
+//               window, one traversal, pairs in no order.
 //   persistent  #SM x occupancy CTAs; warps take windows from an atomic ticket
 //               in Morton order of the window centres (neighbouring windows
 //               share tree paths, so the tree stays in L2); the top tree levels
@@ -348,19 +350,23 @@ __global__ void __launch_bounds__(kPlainWarps * 32)
 __global__ void __launch_bounds__(kPlainWarps * 32)
     plain_write_kernel(TreeView T, WindowView W, int K, int stack_cap,
                        const long long* __restrict__ offsets, int32_t* fid, int32_t* tid,
-                       long long cap, QueryCounters* ctr)
+                       long long cap, const QueryCounters* ctr, int* err)
 {
   extern __shared__ FrontierEntry s_stack[];
   const int warp = threadIdx.x >> 5;
   const long long q = (long long)blockIdx.x * kPlainWarps + warp;
   if (q >= W.n) return;
+  if (ctr->error) {  // the offsets are not to be used
+    raise_error(err, ctr->error);
+    return;
+  }
   if (offsets[W.n] > cap) return;  // overflow: the host reports the required size
   int lg, lc;
   lane_map(T.fanout, lg, lc);
   NodeCache C{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
   OffsetEmit emit{fid, tid, offsets[q], cap, (int)q};
   traverse(T, C, K, lg, lc, W.xmin[q], W.ymin[q], W.xmax[q], W.ymax[q],
-           s_stack + warp * stack_cap, stack_cap, emit, &ctr->error);
+           s_stack + warp * stack_cap, stack_cap, emit, err);
 }
 
 template <bool kContain>
@@ -388,84 +394,89 @@ __global__ void __launch_bounds__(kPlainWarps * 32)
   }
 }
 
-// int64 exclusive scan (counts -> offsets[0..n]), three kernels
+// int64 exclusive scan (counts -> offsets[0..n]) and the result block, one
+// launch: a CTA takes 1024 counts in ticket order and looks back over the
+// tiles before it, 32 at a time (decoupled look-back, one 64-bit status word
+// per tile, zeroed before).  Block sums, their scan, an apply pass and a
+// result kernel, mostly launch latency for the batches of a plain query, took
+// 16 us for 20k windows with the gaps between them; this takes 3.5.
 constexpr int kScanThreads = 1024;
+constexpr unsigned long long kTileAgg = 1ull << 62;
+constexpr unsigned long long kTileIncl = 2ull << 62;
+constexpr unsigned long long kTileFlags = 3ull << 62;
 
-__device__ __forceinline__ long long block_incl_scan(long long v, long long* s_warp)
+__global__ void __launch_bounds__(kScanThreads)
+    scan_kernel(const long long* __restrict__ counts, long long n, long long* __restrict__ offsets,
+                unsigned long long* __restrict__ status, QueryCounters* __restrict__ ctr,
+                long long cap, crt_query_result* __restrict__ res)
 {
+  __shared__ long long s_warp[32];
+  __shared__ long long s_before;
+  __shared__ int s_tile;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) s_tile = (int)atomicAdd(&ctr->ticket, 1ull);
+  __syncthreads();
+  const int tile = s_tile;
+  const long long i = (long long)tile * kScanThreads + threadIdx.x;
+  const long long v = i < n ? counts[i] : 0;
+  long long x = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    long long y = __shfl_up_sync(0xffffffffu, v, o);
-    if (lane >= o) v += y;
+    const long long y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
-  if (lane == 31) s_warp[warp] = v;
+  if (lane == 31) s_warp[warp] = x;
   __syncthreads();
   if (warp == 0) {
-    long long w = lane < (int)(blockDim.x >> 5) ? s_warp[lane] : 0;
+    const long long t = s_warp[lane];
+    long long w = t;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      long long y = __shfl_up_sync(0xffffffffu, w, o);
+      const long long y = __shfl_up_sync(0xffffffffu, w, o);
       if (lane >= o) w += y;
     }
-    s_warp[lane] = w;
+    s_warp[lane] = w - t;
+    const long long total = __shfl_sync(0xffffffffu, w, 31);
+    if (lane == 0) st_relaxed_u64((uint64_t*)&status[tile], (tile ? kTileAgg : kTileIncl) | (uint64_t)total);
+    long long before = 0;
+    uint32_t spins = 0;
+    for (int t0 = tile - 1; t0 >= 0;) {
+      // lane l: tile t0 - l (before tile 0: an inclusive zero)
+      const unsigned long long st = t0 >= lane ? ld_relaxed_u64((const uint64_t*)&status[t0 - lane]) : kTileIncl;
+      const uint32_t open = __ballot_sync(0xffffffffu, (st & kTileFlags) == 0);
+      const uint32_t incl = __ballot_sync(0xffffffffu, (st & kTileFlags) == kTileIncl);
+      // the tiles up to the first inclusive one, if none before it is missing
+      const int stop = incl ? __ffs(incl) : 32;
+      if (open & (stop == 32 ? 0xffffffffu : (1u << stop) - 1)) {
+        if (++spins > kSpinLimit || ld_relaxed_i32(&ctr->error) != 0) {
+          if (lane == 0) raise_error(&ctr->error, CRT_ERR_DEVICE_TIMEOUT);
+          break;
+        }
+        if (spins > 64) __nanosleep(64);
+        continue;
+      }
+      long long part = lane < stop ? (long long)(st & ~kTileFlags) : 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      before += part;
+      if (incl) break;
+      t0 -= 32;
+    }
+    if (lane == 0) {
+      if (tile) st_relaxed_u64((uint64_t*)&status[tile], kTileIncl | (uint64_t)(before + total));
+      s_before = before;
+      if (tile == (int)gridDim.x - 1) {
+        const long long all = before + total;
+        offsets[n] = all;
+        res->required = all;
+        res->overflow = all > cap ? 1 : 0;
+        res->count = all > cap ? 0 : all;
+        res->error = ld_relaxed_i32(&ctr->error);
+      }
+    }
   }
   __syncthreads();
-  if (warp > 0) v += s_warp[warp - 1];
-  __syncthreads();
-  return v;
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    scan_block_sums(const long long* __restrict__ in, long long n, long long* __restrict__ sums)
-{
-  __shared__ long long s_warp[32];
-  long long i = (long long)blockIdx.x * kScanThreads + threadIdx.x;
-  long long v = i < n ? in[i] : 0;
-  v = block_incl_scan(v, s_warp);
-  if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = v;
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    scan_sums_kernel(long long* __restrict__ sums, long long nb)
-{
-  __shared__ long long s_warp[32];
-  __shared__ long long s_tot;
-  long long carry = 0;
-  for (long long b0 = 0; b0 < nb; b0 += kScanThreads) {
-    long long i = b0 + threadIdx.x;
-    long long v = i < nb ? sums[i] : 0;
-    long long x = block_incl_scan(v, s_warp);
-    if (i < nb) sums[i] = carry + x - v;  // exclusive
-    if (threadIdx.x == kScanThreads - 1) s_tot = x;
-    __syncthreads();
-    carry += s_tot;
-    __syncthreads();
-  }
-}
-
-__global__ void __launch_bounds__(kScanThreads)
-    scan_apply_kernel(const long long* __restrict__ in, long long n,
-                      const long long* __restrict__ sums, long long* __restrict__ out)
-{
-  __shared__ long long s_warp[32];
-  long long i = (long long)blockIdx.x * kScanThreads + threadIdx.x;
-  long long v = i < n ? in[i] : 0;
-  long long x = block_incl_scan(v, s_warp);
-  long long base = sums[blockIdx.x];
-  if (i < n) out[i] = base + x - v;
-  if (i == n - 1) out[n] = base + x;
-}
-
-// Writes the result block of a plain query.
-__global__ void plain_result_kernel(const long long* __restrict__ offsets, long long n,
-                                    long long cap, QueryCounters* ctr, crt_query_result* res)
-{
-  long long total = n > 0 ? offsets[n] : 0;
-  res->required = total;
-  res->overflow = total > cap ? 1 : 0;
-  res->count = total > cap ? 0 : total;
-  res->error = ctr->error;
+  if (i < n) offsets[i] = s_before + s_warp[warp] + x - v;
 }
 
 // ---------------------------------------------------------------------------
@@ -713,8 +724,10 @@ constexpr int kSmallSets = 2;     // pairs tested per step, in multiples of K
 constexpr int kPairChunk = 32;  // frontier nodes whose pairs are listed at a time
 
 struct StageEmit {
+  static constexpr bool kCountsTests = false;
   int2* s_out;  // this warp's staging, kSmallStage pairs
   int n = 0;
+  int q = 0;  // the window, where the warp walks one at a time
   int32_t* fid;
   int32_t* tid;
   long long cap;
@@ -788,6 +801,20 @@ struct StageEmit {
       copy_range(bid, __shfl_sync(0xffffffffu, first, src), c, fid, tid, reserve(c), cap,
                  __shfl_sync(0xffffffffu, q, src));
     }
+  }
+  // the emitter of traverse(): every lane's window is q
+  __device__ __forceinline__ void operator()(bool hit, int id)
+  {
+    const uint32_t m = __ballot_sync(0xffffffffu, hit);
+    if (m) hits(m, hit, id, q);
+  }
+  __device__ __forceinline__ void small_ranges(const int* bid, bool mine, long long first, int count)
+  {
+    small_ranges(bid, mine, first, count, q);
+  }
+  __device__ __forceinline__ void big_ranges(const int* bid, bool mine, long long first, long long count)
+  {
+    big_ranges(bid, mine, first, count, q);
   }
 };
 
@@ -991,6 +1018,50 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 3)
   }
   emit.flush();
   if (lane == 0 && emit.total) atomicAdd(&P.ctr->hits, (unsigned long long)emit.total);
+}
+
+// ---------------------------------------------------------------------------
+// Dense form (the drop-in query's small batches)
+// ---------------------------------------------------------------------------
+// One traversal per window in input order, hits staged per warp and flushed
+// densely: no second traversal, no scan, no window order and no compaction, so
+// a batch costs three launches.  The pairs come in no order, which is all the
+// drop-in query promises.  Batches that leave the GPU short of warps give each
+// window kDenseParts of them (Split).
+constexpr int kDenseParts = 8;
+
+__global__ void __launch_bounds__(kPlainWarps * 32)
+    dense_kernel(TreeView T, WindowView W, int K, int stack_cap, int parts, int split_height,
+                 int32_t* fid, int32_t* tid, long long cap, QueryCounters* ctr)
+{
+  extern __shared__ FrontierEntry s_stack[];  // stacks, then kSmallStage pairs per warp
+  const int warp = threadIdx.x >> 5;
+  const long long t = (long long)blockIdx.x * kPlainWarps + warp;
+  const long long q = t / parts;
+  if (q >= W.n) return;
+  Split split;
+  if (parts > 1) {
+    split.part = (int)(t - q * parts);
+    if (*T.lvl_odd == 0) {  // entries carry their height only with the shortcut on
+      split.height = split_height;
+      split.mask = parts - 1;
+    } else if (split.part != 0) {
+      return;
+    }
+  }
+  int lg, lc;
+  lane_map(T.fanout, lg, lc);
+  NodeCache C{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0};
+  StageEmit emit;
+  emit.s_out = s_stack + kPlainWarps * stack_cap + warp * kSmallStage;
+  emit.q = (int)q;
+  emit.fid = fid;
+  emit.tid = tid;
+  emit.cap = cap;
+  emit.next = &ctr->next;
+  traverse(T, C, K, lg, lc, W.xmin[q], W.ymin[q], W.xmax[q], W.ymax[q], s_stack + warp * stack_cap,
+           stack_cap, emit, &ctr->error, 0, 1, split);
+  emit.flush();
 }
 
 // Sorts the recorded holes by start and makes the exclusive prefix of their
@@ -1240,58 +1311,98 @@ LevelTables level_tables(const crt_rtree_f32& rt, int64_t nbox)
   return t;
 }
 
-// Writes the tables (passed by value) to device memory: a one-thread kernel
-// instead of a copy from host memory, so the caller's host thread never waits
-// on a pageable transfer and the write can be recorded in a CUDA graph.
-__global__ void write_levels_kernel(LevelTables t, int* __restrict__ first,
-                                    long long* __restrict__ span)
-{
-  for (int h = threadIdx.x; h < kMaxLevels; h += blockDim.x) {
-    first[h] = t.first[h];
-    span[h] = t.span[h];
-  }
-}
-
-// *odd = 1 when some box is not ordinary (*odd was zeroed before).  Every
-// thread that sees one stores the same value.
+// One launch prepares a query: CTA 0 writes the tables (passed by value, so
+// the host never waits on a pageable transfer and the write can be recorded in
+// a CUDA graph) and the window count, and all CTAs scan the boxes for one that
+// is not ordinary (*odd was zeroed before; every thread that sees one stores
+// the same value).  kVec: the four arrays are 16-byte aligned; eight 16-byte
+// loads per thread are then in flight (10M boxes: 53 us with 4-byte loads, 30
+// so; the read alone takes 25).
+template <bool kVec>
 __global__ void __launch_bounds__(256)
-    odd_boxes_kernel(const float* __restrict__ xmin, const float* __restrict__ ymin,
-                     const float* __restrict__ xmax, const float* __restrict__ ymax, int64_t n,
-                     int* __restrict__ odd)
+    prepare_kernel(LevelTables t, int* __restrict__ first, long long* __restrict__ span,
+                   int* __restrict__ odd, const float* __restrict__ xmin,
+                   const float* __restrict__ ymin, const float* __restrict__ xmax,
+                   const float* __restrict__ ymax, int64_t n, QueryCounters* __restrict__ ctr,
+                   long long nq)
 {
+  if (blockIdx.x == 0) {
+    if (first && threadIdx.x < kMaxLevels) {
+      first[threadIdx.x] = t.first[threadIdx.x];
+      span[threadIdx.x] = t.span[threadIdx.x];
+    }
+    if (ctr && threadIdx.x == 0) ctr->nq = (unsigned long long)nq;
+  }
+  if (n <= 0) return;
   bool bad = false;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  int64_t done = 0;
+  if (kVec) {
+    const auto odd4 = [](float4 a, float4 b) {
+      return !(a.x <= b.x && a.y <= b.y && a.z <= b.z && a.w <= b.w);
+    };
+    const int64_t n4 = n >> 2;
+    for (int64_t i = at; i < n4; i += 2 * stride) {
+      const int64_t j = min(i + stride, n4 - 1);
+      const float4 a0 = reinterpret_cast<const float4*>(xmin)[i], b0 = reinterpret_cast<const float4*>(xmax)[i];
+      const float4 c0 = reinterpret_cast<const float4*>(ymin)[i], d0 = reinterpret_cast<const float4*>(ymax)[i];
+      const float4 a1 = reinterpret_cast<const float4*>(xmin)[j], b1 = reinterpret_cast<const float4*>(xmax)[j];
+      const float4 c1 = reinterpret_cast<const float4*>(ymin)[j], d1 = reinterpret_cast<const float4*>(ymax)[j];
+      bad |= odd4(a0, b0) | odd4(c0, d0) | odd4(a1, b1) | odd4(c1, d1);
+    }
+    done = n4 << 2;
+  }
+  for (int64_t i = done + at; i < n; i += stride)
     bad |= !(xmin[i] <= xmax[i] && ymin[i] <= ymax[i]);
   if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) *odd = 1;
+}
+
+static void launch_prepare(const LevelTables& t, int* first, long long* span, int* odd,
+                           const float* xmin, const float* ymin, const float* xmax,
+                           const float* ymax, int64_t n, QueryCounters* ctr, int64_t nq,
+                           cudaStream_t stream)
+{
+  const bool vec = ((((uintptr_t)xmin) | ((uintptr_t)ymin) | ((uintptr_t)xmax) | ((uintptr_t)ymax)) & 15) == 0;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, vec ? 2048 : 256), (int64_t)sm_count() * 8));
+  if (vec)
+    prepare_kernel<true><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq);
+  else
+    prepare_kernel<false><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq);
+  CRT_LAUNCHED(1);
 }
 
 void launch_odd_boxes(const float* xmin, const float* ymin, const float* xmax, const float* ymax,
                       int64_t n, int* odd, cudaStream_t stream)
 {
   cudaMemsetAsync(odd, 0, sizeof(int), stream);
-  if (n <= 0) return;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), (int64_t)sm_count() * 8));
-  odd_boxes_kernel<<<grid, 256, 0, stream>>>(xmin, ymin, xmax, ymax, n, odd);
-  CRT_LAUNCHED(1);
+  if (n > 0)
+    launch_prepare(LevelTables(), nullptr, nullptr, odd, xmin, ymin, xmax, ymax, n, nullptr, 0, stream);
 }
 
-// Puts the tables at `dev` (kLevelTableBytes, 8-byte aligned), checks the
-// view's boxes for the shortcut and points the view at both.
-static void attach_levels(TreeView& T, const LevelTables& t, void* dev, cudaStream_t stream)
+// Puts the tables at `dev` (kLevelTableBytes, 8-byte aligned, its flag word
+// zeroed by the caller), checks the view's boxes for the shortcut, points the
+// view at both, and sets ctr->nq when ctr is given.
+static void attach_levels(TreeView& T, const LevelTables& t, void* dev, QueryCounters* ctr, int64_t nq,
+                          cudaStream_t stream)
 {
-  if (t.nlev == 0) return;
+  if (t.nlev == 0) {
+    if (ctr) launch_prepare(t, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, ctr, nq, stream);
+    return;
+  }
   int* first = (int*)dev;
   long long* span = (long long*)((char*)dev + sizeof(int) * kMaxLevels);
   int* odd = (int*)((char*)dev + kLevelOddOffset);
-  write_levels_kernel<<<1, 64, 0, stream>>>(t, first, span);
-  CRT_LAUNCHED(1);
-  launch_odd_boxes(T.bxmin, T.bymin, T.bxmax, T.bymax, T.nbox, odd, stream);
+  launch_prepare(t, first, span, odd, T.bxmin, T.bymin, T.bxmax, T.bymax, T.nbox, ctr, nq, stream);
   T.nlev = t.nlev;
   T.lvl_first = first;
   T.lvl_span = span;
   T.lvl_odd = odd;
 }
+
+// Counters and tables, the head of every query's scratch: zeroed in one piece.
+constexpr size_t kHeadTables = 256;
+constexpr size_t kHeadBytes = (kHeadTables + kLevelTableBytes + 255) / 256 * 256;
 
 // Number of levels of a tree with R_sz nodes over nbox boxes at this fanout
 // (1 when the root is the only level).
@@ -1331,13 +1442,14 @@ constexpr int kDefaultChunkRoom = 4096;
 struct PersistVariant {
   int threads;
   int min_blocks;
+  bool share;  // range sharing
   const void* fn;
 };
 
 static const PersistVariant kVariants[] = {
-    {1024, 2, (const void*)persistent_kernel<1024, 2, false>},  // 64 warps/SM, 32 registers
-    {512, 3, (const void*)persistent_kernel<512, 3, false>},    // 48 warps/SM, 40 registers
-    {256, 4, (const void*)persistent_kernel<256, 4, true>},     // 32 warps/SM, 64 registers
+    {1024, 2, false, (const void*)persistent_kernel<1024, 2, false>},  // 64 warps/SM, 32 registers
+    {512, 3, false, (const void*)persistent_kernel<512, 3, false>},    // 48 warps/SM, 40 registers
+    {256, 4, true, (const void*)persistent_kernel<256, 4, true>},     // 32 warps/SM, 64 registers
 };
 
 static const PersistVariant& variant_for(int warps_per_cta)
@@ -1403,7 +1515,7 @@ struct PersistScratch {
 static size_t persist_scratch_bytes(int64_t max_nq, long long max_holes, bool sort)
 {
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-  size_t b = al(sizeof(QueryCounters)) + 2 * al(sizeof(Hole) * max_holes) +
+  size_t b = kHeadBytes + 2 * al(sizeof(Hole) * max_holes) +
              al(sizeof(long long) * (max_holes + 1)) + al(kJobQueueBytes);
   if (sort) b += al(sort_zero_bytes(max_nq)) + 4 * al(4 * (size_t)std::max<int64_t>(max_nq, 1));
   return b;
@@ -1414,7 +1526,7 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
 {
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t off = 0;
-  S.ctr = (QueryCounters*)(base + off); off += al(sizeof(QueryCounters));
+  S.ctr = (QueryCounters*)(base + off); off += kHeadBytes;
   S.holes = (Hole*)(base + off); off += al(sizeof(Hole) * max_holes);
   S.sorted = (Hole*)(base + off); off += al(sizeof(Hole) * max_holes);
   S.cum = (long long*)(base + off); off += al(sizeof(long long) * (max_holes + 1));
@@ -1435,24 +1547,36 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
 }
 
 // A persistent query is three stages on one stream, none synchronising the
-// host: `pre` (reset the counters, order the windows), the traversal kernel,
+// host: `pre` (order the windows; the counters were reset), the traversal kernel,
 // and `post` (sort the unused chunk ends, compact, write the result block).
 // A plan records all three as one CUDA graph.
 static void enqueue_pre(const TreeView& T, const WindowView& W, int64_t max_nq,
-                        const PersistScratch& S, bool sort, bool classes, cudaStream_t stream)
+                        const PersistScratch& S, bool sort, bool classes, bool share,
+                        cudaStream_t stream)
 {
-  // counters (keep nq), the job queue's ready flags and the sort's zeroed block
-  cudaMemsetAsync(S.ctr, 0, offsetof(QueryCounters, nq), stream);
-  cudaMemsetAsync(S.jobs, 0, kJobQueueBytes, stream);
-  if (sort && max_nq > 0) {
+  // the job queue's ready flags (where ranges are shared) and the sort's zeroed
+  // block, which follows them
+  const bool order = sort && max_nq > 0;
+  char* z0 = share ? (char*)S.jobs : (char*)S.sort_zero;
+  char* z1 = order ? (char*)S.sort_zero + sort_zero_bytes(max_nq) : (char*)S.jobs + kJobQueueBytes;
+  if (share || order) cudaMemsetAsync(z0, 0, (size_t)(z1 - z0), stream);
+  if (order) {
     const int sms = sm_count();
-    cudaMemsetAsync(S.sort_zero, 0, sort_zero_bytes(max_nq), stream);
     int g = (int)std::min<int64_t>(cdiv(max_nq, 256), (int64_t)sms * 4);
     window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, T, classes, S.ctr, S.cols.key[0],
                                                           sort_ctrl(S.sort_zero));
     sort_passes(S.cols, W.n, kDigits, S.sort_zero, stream);
     CRT_LAUNCHED(1);
   }
+}
+
+// Nodes of this height are dealt out among the warps sharing a window: the
+// first height whose nodes hold 256 boxes, at most the root's children's.
+static int split_height(const TreeView& T)
+{
+  int h = 0;
+  for (int64_t span = T.fanout; span < 256 && h < T.nlev - 2; span *= T.fanout) h++;
+  return h;
 }
 
 struct TraverseLaunch {
@@ -1494,9 +1618,7 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
   P.stage_n = ps.stage_n;
   P.parts = parts;
   P.classes = window_classes(T, sort);
-  P.split_height = 0;  // the first height whose nodes hold 256 boxes, at most the root's children's
-  for (int64_t span = T.fanout; span < 256 && P.split_height < T.nlev - 2; span *= T.fanout)
-    P.split_height++;
+  P.split_height = split_height(T);
   P.chunk = chunk;
   P.fid = fid;
   P.tid = tid;
@@ -1595,6 +1717,106 @@ static int window_parts(const crt_query_opts& o)
   return (w == 1 || w == 2 || w == 4) ? w : -1;
 }
 
+// Whether the dense form's shared memory fits a CTA (it stages pairs beside
+// the stacks; a fanout in the thousands leaves no room).
+static size_t dense_smem(int stack_cap)
+{
+  return (size_t)kPlainWarps * (stack_cap + kSmallStage) * sizeof(FrontierEntry);
+}
+bool query_dense_fits(int64_t nbox, int fanout)
+{
+  return dense_smem(traversal_shape(nbox, fanout).stack_cap) <= 227 * 1024;
+}
+
+// The dense form into caller-owned columns of `cap` slots each: *pairs is the
+// pair count, more than cap when the output was too small (nothing past it is
+// written).  Synchronises the stream.
+int query_dense(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,
+                int32_t* fid, int32_t* tid, int64_t cap, int64_t* pairs, cudaStream_t stream)
+{
+  NvtxRange range("crt_query_dense");
+  *pairs = 0;
+  if (qbox.sz <= 0) return CRT_OK;
+  TreeView T = make_view(rt, rbox);
+  WindowView W{qbox.xmin, qbox.ymin, qbox.xmax, qbox.ymax, qbox.sz};
+  const TraversalShape sh = traversal_shape(rbox.sz, rt.fanout);
+  char* scr = nullptr;
+  if (cudaMallocAsync((void**)&scr, kHeadBytes, stream) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CRT_ERR_OOM, "query: scratch allocation failed");
+  }
+  QueryCounters* ctr = (QueryCounters*)scr;
+  cudaMemsetAsync(scr, 0, kHeadBytes, stream);
+  attach_levels(T, level_tables(rt, rbox.sz), scr + kHeadTables, nullptr, 0, stream);
+  // kPlainWarps x 4 warps per SM is what the traversal's shared memory allows
+  const bool few = T.nlev > 1 && W.n * kDenseParts <= (int64_t)sm_count() * kPlainWarps * 4;
+  const int parts = few ? kDenseParts : 1;
+  const size_t smem = dense_smem(sh.stack_cap);
+  cudaFuncSetAttribute(dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  {
+    ProfScope ps("traverse_dense", stream);
+    dense_kernel<<<(unsigned)cdiv(W.n * parts, kPlainWarps), kPlainWarps * 32, smem, stream>>>(
+        T, W, sh.K, sh.stack_cap, parts, split_height(T), fid, tid, cap, ctr);
+    CRT_LAUNCHED(1);
+  }
+  QueryCounters h{};
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ctr, sizeof(h), cudaMemcpyDeviceToHost, stream);
+  cudaFreeAsync(scr, stream);
+  const cudaError_t es = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess) e = es;
+  if (e != cudaSuccess) return cuda_fail(e, "query");
+  if (h.error) return fail(h.error, "query: device-side error");
+  *pairs = (int64_t)h.next;
+  return CRT_OK;
+}
+
+// Scratch of a plain query: the head (counters and tables) and behind it the
+// scan's status words, one count per window, the offsets.
+struct PlainScratch {
+  char* head;
+  unsigned long long* status;
+  long long* counts;
+  long long* offsets;
+};
+constexpr int64_t plain_tiles(int64_t nq) { return nq < 1 ? 1 : (nq + kScanThreads - 1) / kScanThreads; }
+// Bytes of the head and the status words, zeroed together.
+constexpr size_t plain_zero_bytes(int64_t nq)
+{
+  return (kHeadBytes + 8 * (size_t)plain_tiles(nq) + 255) / 256 * 256;
+}
+
+// The plain query's launches: reset, prepare, count, scan (with the result
+// block), write.
+static void enqueue_plain(TreeView T, const LevelTables& lt, const WindowView& W, const PlainScratch& S,
+                          int32_t* fid, int32_t* tid, int64_t capacity, crt_query_result* res,
+                          cudaStream_t stream)
+{
+  const TraversalShape sh = traversal_shape(T.nbox, T.fanout);
+  QueryCounters* ctr = (QueryCounters*)S.head;
+  const int64_t nq = W.n;
+  cudaMemsetAsync(S.head, 0, plain_zero_bytes(nq), stream);
+  attach_levels(T, lt, S.head + kHeadTables, nullptr, 0, stream);
+  const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
+  cudaFuncSetAttribute(plain_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(plain_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const unsigned g = (unsigned)cdiv(nq, kPlainWarps);
+  if (nq > 0) {
+    ProfScope ps("traverse_plain", stream);
+    plain_count_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap, S.counts, ctr);
+    CRT_LAUNCHED(1);
+  }
+  scan_kernel<<<(unsigned)plain_tiles(nq), kScanThreads, 0, stream>>>(
+      S.counts, nq, S.offsets, S.status, ctr, capacity, res);
+  CRT_LAUNCHED(1);
+  if (nq > 0) {
+    ProfScope ps("traverse_plain", stream);
+    plain_write_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap, S.offsets, fid,
+                                                              tid, capacity, ctr, &res->error);
+    CRT_LAUNCHED(1);
+  }
+}
+
 int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,
                int32_t* fid, int32_t* tid, int64_t capacity, crt_query_result* d_result,
                int64_t* d_offsets, const crt_query_opts& opts, cudaStream_t stream)
@@ -1612,49 +1834,21 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   const LevelTables lt = opts.no_contain ? LevelTables() : level_tables(rt, rbox.sz);
   WindowView W{qbox.xmin, qbox.ymin, qbox.xmax, qbox.ymax, qbox.sz};
   const int64_t nq = qbox.sz;
-  const TraversalShape sh = traversal_shape(rbox.sz, rt.fanout);
-  const int sms = sm_count();
 
   if (opts.mode == CRT_QUERY_PLAIN) {
-    // scratch: counters, counts, block sums (+ offsets when the caller gave none)
-    const int64_t nb = std::max<int64_t>(1, cdiv(nq, kScanThreads));
-    size_t bytes = 256 + 8 * (size_t)std::max<int64_t>(nq, 1) + 8 * (size_t)nb + 256 +
-                   (d_offsets ? 0 : 8 * (size_t)(nq + 1) + 256) + kLevelTableBytes + 256;
+    const size_t zero = plain_zero_bytes(nq);
+    const size_t per = 8 * (size_t)(nq + 1);
     char* scr = nullptr;
-    if (cudaMallocAsync((void**)&scr, bytes, stream) != cudaSuccess) {
+    if (cudaMallocAsync((void**)&scr, zero + (d_offsets ? 1 : 2) * per, stream) != cudaSuccess) {
       cudaGetLastError();
       return fail(CRT_ERR_OOM, "query: scratch allocation failed");
     }
-    QueryCounters* ctr = (QueryCounters*)scr;
-    long long* counts = (long long*)(scr + 256);
-    long long* sums = counts + std::max<int64_t>(nq, 1);
-    long long* offsets = d_offsets ? (long long*)d_offsets : sums + nb + 32;
-    char* tables = (char*)(((uintptr_t)(scr + bytes - kLevelTableBytes - 256) + 255) & ~(uintptr_t)255);
-    attach_levels(T, lt, tables, stream);
-    cudaMemsetAsync(ctr, 0, sizeof(QueryCounters), stream);
-    cudaMemsetAsync(offsets, 0, 8, stream);
-    const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-    cudaFuncSetAttribute(plain_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(plain_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (nq > 0) {
-      const unsigned g = (unsigned)cdiv(nq, kPlainWarps);
-      {
-        ProfScope ps("traverse_plain", stream);
-        plain_count_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap, counts,
-                                                                  ctr);
-      }
-      scan_block_sums<<<(unsigned)nb, kScanThreads, 0, stream>>>(counts, nq, sums);
-      scan_sums_kernel<<<1, kScanThreads, 0, stream>>>(sums, nb);
-      scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(counts, nq, sums, offsets);
-      {
-        ProfScope ps("traverse_plain", stream);
-        plain_write_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap,
-                                                                  offsets, fid, tid, capacity, ctr);
-      }
-      CRT_LAUNCHED(5);
-    }
-    plain_result_kernel<<<1, 1, 0, stream>>>(offsets, nq, capacity, ctr, d_result);
-    CRT_LAUNCHED(1);
+    PlainScratch S;
+    S.head = scr;
+    S.status = (unsigned long long*)(scr + kHeadBytes);
+    S.counts = (long long*)(scr + zero);
+    S.offsets = d_offsets ? (long long*)d_offsets : (long long*)(scr + zero + per);
+    enqueue_plain(T, lt, W, S, fid, tid, capacity, d_result, stream);
     cudaFreeAsync(scr, stream);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "query (plain)");
@@ -1662,6 +1856,7 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   }
 
   // persistent
+  const TraversalShape sh = traversal_shape(rbox.sz, rt.fanout);
   const bool sort = opts.sort_windows != 0 && nq > 1;
   const int stage_n = fit_stage_nodes(rt, rbox.sz, opts.stage_levels, sh.stack_cap,
                                       opts.warps_per_cta);
@@ -1671,7 +1866,7 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   if (!persist_shape(sh.stack_cap, stage_n, opts.warps_per_cta).v)
     return fail(CRT_ERR_NOT_SUPPORTED, "query: traversal stack too large");
   const long long max_holes = max_holes_for(sh.stack_cap, stage_n, opts.warps_per_cta);
-  const size_t bytes = persist_scratch_bytes(nq, max_holes, sort) + kLevelTableBytes;
+  const size_t bytes = persist_scratch_bytes(nq, max_holes, sort);
   char* scr = nullptr;
   if (cudaMallocAsync((void**)&scr, bytes, stream) != cudaSuccess) {
     cudaGetLastError();
@@ -1679,10 +1874,9 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   }
   PersistScratch S;
   persist_scratch_carve(scr, nq, max_holes, sort, S);
-  attach_levels(T, lt, scr + S.bytes, stream);
-  set_nq_kernel<<<1, 1, 0, stream>>>(S.ctr, nq);
-  CRT_LAUNCHED(1);
-  enqueue_pre(T, W, nq, S, sort, window_classes(T, sort), stream);
+  cudaMemsetAsync(scr, 0, kHeadBytes, stream);
+  attach_levels(T, lt, scr + kHeadTables, S.ctr, nq, stream);
+  enqueue_pre(T, W, nq, S, sort, window_classes(T, sort), variant_for(opts.warps_per_cta).share, stream);
   cudaError_t e = launch_traverse(make_traverse(T, W, S, sort, stage_n, fid, tid, capacity, chunk,
                                                 opts.warps_per_cta, parts),
                                   stream);
@@ -1691,7 +1885,6 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   if (e == cudaSuccess) e = cudaGetLastError();
   else cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "query (persistent)");
-  (void)sms;
   return CRT_OK;
 }
 
@@ -1715,12 +1908,10 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
 // overlaps on the GPU (different streams, or another thread) race on it and
 // must be serialised by the caller.
 constexpr int64_t kNoAllocMaxWindows = 1 << 16;
-constexpr size_t kNoAllocCountsOff = 256;
-constexpr size_t kNoAllocSumsOff = kNoAllocCountsOff + 8 * (size_t)kNoAllocMaxWindows;
-constexpr size_t kNoAllocOffsetsOff = kNoAllocSumsOff + 8 * 256;
-constexpr size_t kNoAllocTablesOff =
+constexpr size_t kNoAllocCountsOff = plain_zero_bytes(kNoAllocMaxWindows);
+constexpr size_t kNoAllocOffsetsOff = kNoAllocCountsOff + 8 * (size_t)kNoAllocMaxWindows;
+constexpr size_t kNoAllocBytes =
     (kNoAllocOffsetsOff + 8 * (size_t)(kNoAllocMaxWindows + 1) + 255) / 256 * 256;
-constexpr size_t kNoAllocBytes = kNoAllocTablesOff + (kLevelTableBytes + 255) / 256 * 256;
 static_assert(kNoAllocBytes <= (1u << 20) + 4096, "no-alloc scratch stays near 1 MiB");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -1764,32 +1955,13 @@ int query_plain_noalloc(const crt_rtree_f32& rt, const crt_bbox_f32& rbox,
   int rc = noalloc_scratch_address(&scr);
   if (rc != CRT_OK) return rc;
   TreeView T = make_view(rt, rbox);
-  attach_levels(T, level_tables(rt, rbox.sz), scr + kNoAllocTablesOff, stream);
   WindowView W{qbox.xmin, qbox.ymin, qbox.xmax, qbox.ymax, qbox.sz};
-  const int64_t nq = qbox.sz;
-  const TraversalShape sh = traversal_shape(rbox.sz, rt.fanout);
-  QueryCounters* ctr = (QueryCounters*)scr;
-  long long* counts = (long long*)(scr + kNoAllocCountsOff);
-  long long* sums = (long long*)(scr + kNoAllocSumsOff);
-  long long* offsets = (long long*)(scr + kNoAllocOffsetsOff);
-  const int64_t nb = std::max<int64_t>(1, cdiv(nq, kScanThreads));
-  cudaMemsetAsync(ctr, 0, sizeof(QueryCounters), stream);
-  cudaMemsetAsync(offsets, 0, 8, stream);
-  const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-  cudaFuncSetAttribute(plain_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(plain_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (nq > 0) {
-    const unsigned g = (unsigned)cdiv(nq, kPlainWarps);
-    plain_count_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap, counts, ctr);
-    scan_block_sums<<<(unsigned)nb, kScanThreads, 0, stream>>>(counts, nq, sums);
-    scan_sums_kernel<<<1, kScanThreads, 0, stream>>>(sums, nb);
-    scan_apply_kernel<<<(unsigned)nb, kScanThreads, 0, stream>>>(counts, nq, sums, offsets);
-    plain_write_kernel<<<g, kPlainWarps * 32, smem, stream>>>(T, W, sh.K, sh.stack_cap, offsets,
-                                                              fid, tid, capacity, ctr);
-    CRT_LAUNCHED(5);
-  }
-  plain_result_kernel<<<1, 1, 0, stream>>>(offsets, nq, capacity, ctr, d_result);
-  CRT_LAUNCHED(1);
+  PlainScratch S;
+  S.head = scr;
+  S.status = (unsigned long long*)(scr + kHeadBytes);
+  S.counts = (long long*)(scr + kNoAllocCountsOff);
+  S.offsets = (long long*)(scr + kNoAllocOffsetsOff);
+  enqueue_plain(T, level_tables(rt, rbox.sz), W, S, fid, tid, capacity, d_result, stream);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "query_plain_noalloc");
   return CRT_OK;
@@ -1808,7 +1980,7 @@ int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   }
   QueryCounters* ctr = (QueryCounters*)scr;
   unsigned long long* tot = (unsigned long long*)(scr + 256);  // [3] box-by-box, [3] containment
-  cudaMemsetAsync(scr, 0, 1024, stream);
+  cudaMemsetAsync(scr, 0, 1024 + kLevelTableBytes, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
   cudaFuncSetAttribute(stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaFuncSetAttribute(stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1819,7 +1991,7 @@ int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
         T, W, sh.K, sh.stack_cap, (long long*)d_hits, (long long*)d_tested, tot, ctr);
     // this library's: contained subtrees are emitted by slot range
     TreeView Tc = T;
-    attach_levels(Tc, level_tables(rt, rbox.sz), scr + 1024, stream);
+    attach_levels(Tc, level_tables(rt, rbox.sz), scr + 1024, nullptr, 0, stream);
     stats_kernel<true><<<g, kPlainWarps * 32, smem, stream>>>(Tc, W, sh.K, sh.stack_cap, nullptr,
                                                               nullptr, tot + 3, ctr);
     CRT_LAUNCHED(2);
@@ -1918,17 +2090,16 @@ int plan_create(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
     return fail(CRT_ERR_NOT_SUPPORTED, "plan: traversal stack too large");
   }
   const long long max_holes = max_holes_for(sh.stack_cap, p->stage_n, opts.warps_per_cta);
-  const size_t bytes = persist_scratch_bytes(max_nq, max_holes, p->sort) + kLevelTableBytes;
+  const size_t bytes = persist_scratch_bytes(max_nq, max_holes, p->sort);
   if (cudaMalloc((void**)&p->scratch, bytes) != cudaSuccess) {
     cudaGetLastError();
     delete p;
     return fail(CRT_ERR_OOM, "plan: scratch allocation failed");
   }
   persist_scratch_carve(p->scratch, max_nq, max_holes, p->sort, p->S);
-  if (!opts.no_contain) attach_levels(p->T, level_tables(rt, rbox.sz), p->scratch + p->S.bytes, stream);
-  cudaMemsetAsync(p->S.ctr, 0, sizeof(QueryCounters), stream);
-  set_nq_kernel<<<1, 1, 0, stream>>>(p->S.ctr, max_nq);
-  CRT_LAUNCHED(1);
+  cudaMemsetAsync(p->scratch, 0, kHeadBytes, stream);
+  attach_levels(p->T, opts.no_contain ? LevelTables() : level_tables(rt, rbox.sz),
+                p->scratch + kHeadTables, p->S.ctr, max_nq, stream);
   p->traverse = make_traverse(p->T, p->W, p->S, p->sort, p->stage_n, fid, tid, capacity, p->chunk,
                               opts.warps_per_cta, parts);
   // capture the whole query on a private stream; a window-sorting plan
@@ -1941,7 +2112,10 @@ int plan_create(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   if (e == cudaSuccess) e = cudaEventCreate(&p->own[1]);
   if (e == cudaSuccess) e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    enqueue_pre(p->T, p->W, max_nq, p->S, p->sort, window_classes(p->T, p->sort), cs);
+    // each replay resets the counters (nq stays)
+    cudaMemsetAsync(p->S.ctr, 0, offsetof(QueryCounters, nq), cs);
+    enqueue_pre(p->T, p->W, max_nq, p->S, p->sort, window_classes(p->T, p->sort),
+                variant_for(opts.warps_per_cta).share, cs);
     cudaError_t le = cudaEventRecordWithFlags(p->own[0], cs, cudaEventRecordExternal);
     if (le == cudaSuccess) le = launch_traverse(p->traverse, cs);
     if (le == cudaSuccess) le = cudaEventRecordWithFlags(p->own[1], cs, cudaEventRecordExternal);

@@ -122,3 +122,42 @@ def test_options_beside_classes(crt, opts):
     rng = np.random.default_rng(8)
     b = D.uniform_boxes(40_000, seed=8)
     check(crt, b, windows(rng, 1500, SMALL + LARGE + HUGE), 10, **opts)
+
+
+@pytest.mark.parametrize("fanout", [2, 10, 16, 40])
+@pytest.mark.parametrize("odd", [False, True])
+def test_small_drop_in_batches(crt, fanout, odd):
+    """Batches around the line where several warps share a window (148 * 32 / 8
+    windows), on boxes that are all ordinary and on a set that is not, a
+    batch of many pairs after one of few (the output is sized from the last)."""
+    rng = np.random.default_rng(fanout)
+    b = D.clustered_boxes(50_021, seed=fanout)
+    if odd:
+        b.xmax[77] = np.nan
+        b.xmin[99], b.xmax[99] = b.xmax[99] + 3, b.xmin[99]
+    d = crt.BBox.from_host(b)
+    rt = crt.RTree(fanout)
+    crt.build_rtree(d, rt)
+    sb, t = O.build(b, fanout)
+    for nq, sides in ((5000, SMALL), (1, HUGE), (592, SMALL + LARGE + HUGE), (593, SMALL + LARGE),
+                      (40, LARGE), (16, SMALL)):
+        q = windows(rng, nq, sides)
+        pairs = crt.bfs_frontier(rt, d, crt.BBox.from_host(q))
+        got = O.canonical_pairs(*pairs.to_host())
+        want = O.canonical_pairs(*O.tree_query_pairs(t, sb, q))
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]), (nq, fanout)
+        pairs.free()
+
+
+@pytest.mark.parametrize("nq", [1, 7, 8, 8191, 8192, 8193, 65_536, 65_537])
+def test_plain_offsets_at_scan_edges(crt, nq):
+    """Plain offsets around the one-CTA scan's tile and its limit."""
+    rng = np.random.default_rng(nq)
+    b = D.uniform_boxes(5_003, seed=3)
+    q = windows(rng, nq, (0.0, 1e-3, 2e-2))
+    d, rt = crt.build_into(crt.BBox.from_host(b), 10)
+    fid, tid, offs = crt.query(rt, d, crt.BBox.from_host(q), mode=crt.CRT_QUERY_PLAIN)
+    sb, t = O.build(b, 10)
+    counts = O.tree_query_stats(t, sb, q).counts
+    assert np.array_equal(offs.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
+    assert np.array_equal(tid.cpu().numpy(), np.repeat(np.arange(nq), counts))
