@@ -5,10 +5,10 @@
 //                  flipped 32-bit Morton key and the slot of a 32-byte AoS
 //                  record of each box (records of a 4096-box tile grouped by
 //                  the key's top digit), and count all four 8-bit key digits.
-//   2. plan        one CTA: which digit passes are non-uniform (a uniform digit
-//                  leaves a stable order unchanged, so its pass is skipped) and
-//                  the global bucket start of every digit value.
-//   3. 4 x onesweep  stable LSD radix passes over (key, slot) with decoupled
+//   2. plan        the encoder's last CTA: which digit passes are non-uniform (a
+//                  uniform digit leaves a stable order unchanged, so its pass is
+//                  skipped) and the global bucket start of every digit value.
+//   3. 4 x sweep    (sort.cu) stable LSD radix passes over (key, slot) with decoupled
 //                  look-back across tiles: one read and one write of the pairs
 //                  per pass.  The first active pass reads the encoder's slots,
 //                  the last one writes only slots.
@@ -16,7 +16,8 @@
 //                  tile, so lines are shared by neighbouring records), write the permuted
 //                  SoA, and reduce every run of `fanout` boxes into its
 //                  leaf-parent node.
-//   5. upper levels  reduce runs of `fanout` nodes, level by level up to the root.
+//   5. upper levels  reduce runs of `fanout` nodes, up to the root: a launch that
+//                  fits one wave makes every level above its own.
 // Node order, pos and len follow the reference exactly (root at 0, levels
 // downward, children contiguous, leaf-parent pos = R_sz + first slot).
 #include <cuda_runtime.h>
@@ -194,6 +195,7 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(BoxIn in, int64_t n
     }
     __syncthreads();
   }
+  chain_next();
   for (int i = tid; i < kDigits * kBins; i += kEncThreads) {
     const uint32_t v = (&sh[0][0])[i];
     if (v) atomicAdd(&ctrl->hist[i], v);
@@ -206,32 +208,89 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(BoxIn in, int64_t n
 // ---------------------------------------------------------------------------
 constexpr int kLevelThreads = 256;
 constexpr int kLevelChunk = 2048;  // children staged per round
+constexpr int kUpMax = 12;         // levels a CTA makes above its own parents
+constexpr int kTailMax = 32;       // levels the last CTA makes
+constexpr int64_t kTailNodes = 16384;  // most children it starts from
+
+struct NodeOut {
+  float* __restrict__ xmin;
+  float* __restrict__ ymin;
+  float* __restrict__ xmax;
+  float* __restrict__ ymax;
+  int* __restrict__ pos;
+  int* __restrict__ len;
+};
+
+// One launch of the level kernel: a level of nparent parents over nchild
+// children, the up_n levels above it that each CTA makes from its own parents,
+// and the tail_n levels above those that the last CTA to finish makes alone.
+struct LevelArgs {
+  int nodes_per_cta;  // a multiple of fanout^up_n
+  int fanout;
+  int64_t nchild, nparent;
+  int parent_start;  // first node of the parents' level
+  int pos_base;      // pos of the first parent
+  int child_start;   // first node of the children's level (inner levels)
+  int up_n;
+  int up_start[kUpMax];
+  int tail_n;
+  int tail_child;        // first node and node count of the level below the tail
+  int tail_nchild;
+  int tail_start[kTailMax];
+  int* done;  // CTAs finished (zeroed)
+};
+
+__device__ __forceinline__ void put_node(const NodeOut& N, int o, float4 m, int pos, int len)
+{
+  N.xmin[o] = m.x;
+  N.ymin[o] = m.y;
+  N.xmax[o] = m.z;
+  N.ymax[o] = m.w;
+  N.pos[o] = pos;
+  N.len[o] = len;
+}
+
+// reduce_op (src/rtree_bulkload_thrust.cuh:38-50) of one more child.
+__device__ __forceinline__ float4 merge_box(float4 a, float4 m)
+{
+  return make_float4(fminf(a.x, m.x), fminf(a.y, m.y), fmaxf(a.z, m.z), fmaxf(a.w, m.w));
+}
 
 // Reduces runs of `fanout` consecutive children into parent nodes
 // (reduce_op, src/rtree_bulkload_thrust.cuh:38-50: min, min, max, max of the
 // MBR, first child index, child count).  kLeaf: children are the sorted boxes,
 // gathered from the AoS copy through the sorted slot order, and the permuted
 // SoA is written on the way; otherwise children are nodes at child_start.
-template <bool kLeaf>
+// The leaf level is bound by its gathers: 100M clustered boxes take 2.1 ms, and
+// 0.86 with the records read in order; within windows of 32 MB (they fit the
+// L2 and few TLB entries) the same gathers take 1.2 ms.  Tile shapes, records
+// per thread in flight and 32-byte loads measured no difference.  A level above
+// it is a few microseconds of launch and latency, so a CTA goes on upwards over
+// the parents it holds in shared memory, and the last CTA makes the top of the
+// tree: one or two launches instead of one per level (all levels of 20k boxes,
+// fanout 10: 19 us with the gaps between the launches, 10 now; 1M: 37, now 25).
+//
+// kFuse: the launch makes the levels above its own too.
+template <bool kLeaf, bool kFuse>
 __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs per SM
-    level_kernel(int nodes_per_cta, int fanout, int64_t nchild, int64_t nparent,
-                 int64_t parent_start, int64_t pos_base,
+    level_kernel(LevelArgs A, NodeOut N,
                  // leaf inputs/outputs
                  const uint32_t* __restrict__ vals0, const uint32_t* __restrict__ vals1,
                  const SortCtrl* __restrict__ ctrl, const Box32* __restrict__ aos,
                  float* __restrict__ oxmin, float* __restrict__ oymin,
-                 float* __restrict__ oxmax, float* __restrict__ oymax, int* __restrict__ oid,
-                 // node arrays
-                 float* __restrict__ nxmin, float* __restrict__ nymin,
-                 float* __restrict__ nxmax, float* __restrict__ nymax, int* __restrict__ npos,
-                 int* __restrict__ nlen, int64_t child_start)
+                 float* __restrict__ oxmax, float* __restrict__ oymax, int* __restrict__ oid)
 {
   __shared__ float4 s_mbr[kLevelChunk];
-  const int64_t p0 = (int64_t)blockIdx.x * nodes_per_cta;
-  const int64_t p1 = min(nparent, p0 + nodes_per_cta);
-  if (p0 >= p1) return;
-  const int64_t c0 = p0 * fanout;
-  const int64_t c1 = min(nchild, p1 * fanout);
+  __shared__ int s_last;
+  chain_wait();
+  // 32-bit indices: children and parents are below 2^31, their sums with a
+  // fanout below 2^32
+  const uint32_t fanout = (uint32_t)A.fanout;
+  const uint32_t nchild = (uint32_t)A.nchild;
+  const uint32_t p0 = blockIdx.x * (uint32_t)A.nodes_per_cta;
+  const uint32_t p1 = min((uint32_t)A.nparent, p0 + (uint32_t)A.nodes_per_cta);
+  const uint32_t c0 = p0 * fanout;
+  const uint32_t c1 = min(nchild, p1 * fanout);
   const uint32_t* sorted = nullptr;
   if (kLeaf) {
     // record slots in sorted order (the encoder's slots when no pass ran)
@@ -239,14 +298,14 @@ __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs
     sorted = (na & 1) ? vals1 : vals0;
   }
   // this thread's parent (if any) and its child range
-  const int64_t my = p0 + threadIdx.x;
+  const uint32_t my = p0 + threadIdx.x;
   const bool have = my < p1;
-  const int64_t my_c0 = my * fanout;
-  const int64_t my_c1 = min(nchild, my_c0 + fanout);
-  float a = 0.f, b = 0.f, c = 0.f, d = 0.f;
+  const uint32_t my_c0 = my * fanout;
+  const uint32_t my_c1 = min(nchild, my_c0 + fanout);
+  float4 box = make_float4(0.f, 0.f, 0.f, 0.f);
   bool init = false;
-  for (int64_t cb = c0; cb < c1; cb += kLevelChunk) {
-    const int64_t ce = min(c1, cb + (int64_t)kLevelChunk);
+  for (uint32_t cb = c0; cb < c1; cb += kLevelChunk) {
+    const uint32_t ce = min(c1, cb + (uint32_t)kLevelChunk);
     if (kLeaf) {
       // all slot loads, then all 32-byte record loads, then the stores: each
       // thread keeps kGather record reads in flight
@@ -254,9 +313,9 @@ __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs
       uint32_t src[kGather];
 #pragma unroll
       for (int u = 0; u < kGather; u++) {
-        const int64_t s = cb + threadIdx.x + u * kLevelThreads;
+        const uint32_t s = cb + threadIdx.x + u * kLevelThreads;
         src[u] = s < ce ? sorted[s] : 0u;
-        if ((int64_t)src[u] >= nchild) src[u] = s < ce ? (uint32_t)s : 0u;  // only after a sort error (reported)
+        if (src[u] >= nchild) src[u] = s < ce ? s : 0u;  // only after a sort error (reported)
       }
       Box32 bx[kGather];
 #pragma unroll
@@ -264,7 +323,7 @@ __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs
         if (cb + threadIdx.x + u * kLevelThreads < ce) bx[u] = aos[src[u]];
 #pragma unroll
       for (int u = 0; u < kGather; u++) {
-        const int64_t s = cb + threadIdx.x + u * kLevelThreads;
+        const uint32_t s = cb + threadIdx.x + u * kLevelThreads;
         if (s < ce) {
           const float4 m = bx[u].mbr;
           __stcs(oxmin + s, m.x);
@@ -276,37 +335,78 @@ __global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs
         }
       }
     } else {
-      for (int64_t s = cb + threadIdx.x; s < ce; s += kLevelThreads) {
-        const int64_t i = child_start + s;
-        s_mbr[s - cb] = make_float4(nxmin[i], nymin[i], nxmax[i], nymax[i]);
+      for (uint32_t s = cb + threadIdx.x; s < ce; s += kLevelThreads) {
+        const uint32_t i = (uint32_t)A.child_start + s;
+        s_mbr[s - cb] = make_float4(N.xmin[i], N.ymin[i], N.xmax[i], N.ymax[i]);
       }
     }
     __syncthreads();
     if (have) {
-      const int64_t lo = max(my_c0, cb), hi = min(my_c1, ce);
-      for (int64_t s = lo; s < hi; s++) {
-        float4 m = s_mbr[s - cb];
-        if (!init) {
-          a = m.x; b = m.y; c = m.z; d = m.w;
-          init = true;
-        } else {
-          a = fminf(a, m.x);
-          b = fminf(b, m.y);
-          c = fmaxf(c, m.z);
-          d = fmaxf(d, m.w);
-        }
+      const uint32_t lo = max(my_c0, cb), hi = min(my_c1, ce);
+      for (uint32_t s = lo; s < hi; s++) {
+        const float4 m = s_mbr[s - cb];
+        box = init ? merge_box(box, m) : m;
+        init = true;
       }
     }
     __syncthreads();
   }
-  if (have) {
-    const int64_t o = parent_start + my;
-    nxmin[o] = a;
-    nymin[o] = b;
-    nxmax[o] = c;
-    nymax[o] = d;
-    npos[o] = (int)(pos_base + my_c0);
-    nlen[o] = (int)(my_c1 - my_c0);
+  if (have)
+    put_node(N, (int)(A.parent_start + my), box, (int)(A.pos_base + my_c0), (int)(my_c1 - my_c0));
+  chain_next();
+  if constexpr (!kFuse) return;
+  // the levels above, over this CTA's parents
+  if (A.up_n > 0) {
+    if (have) s_mbr[threadIdx.x] = box;
+    int cnt = (int)(p1 - p0);
+    int first = (int)p0;  // index in its level of the CTA's first node
+    int below = A.parent_start;
+    for (int k = 0; k < A.up_n; k++) {
+      __syncthreads();
+      const int np = (cnt + (int)fanout - 1) / (int)fanout;
+      const int lo = (int)threadIdx.x * (int)fanout, hi = min(cnt, lo + (int)fanout);
+      float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+      if ((int)threadIdx.x < np) {
+        m = s_mbr[lo];
+        for (int i = lo + 1; i < hi; i++) m = merge_box(m, s_mbr[i]);
+      }
+      __syncthreads();
+      if ((int)threadIdx.x < np) {
+        s_mbr[threadIdx.x] = m;
+        put_node(N, (int)(A.up_start[k] + first / (int)fanout + (int)threadIdx.x), m, (int)(below + first + lo),
+                 hi - lo);
+      }
+      first /= (int)fanout;
+      below = A.up_start[k];
+      cnt = np;
+    }
+  }
+  // the top of the tree, by the CTA that finishes last
+  if (A.tail_n > 0) {
+    __threadfence();  // this thread's nodes before the count
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(A.done, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    int below = A.tail_child, cnt = A.tail_nchild;
+    for (int k = 0; k < A.tail_n; k++) {
+      const int np = (cnt + (int)fanout - 1) / (int)fanout;
+      for (int p = threadIdx.x; p < np; p += kLevelThreads) {
+        const int lo = p * (int)fanout, hi = min(cnt, lo + (int)fanout);
+        const auto child = [&](int i) {  // another CTA's, or written a level ago: through L2
+          const int j = below + i;
+          return make_float4(__ldcg(N.xmin + j), __ldcg(N.ymin + j), __ldcg(N.xmax + j), __ldcg(N.ymax + j));
+        };
+        float4 m = child(lo);
+#pragma unroll 4
+        for (int i = lo + 1; i < hi; i++) m = merge_box(m, child(i));
+        put_node(N, A.tail_start[k] + p, m, below + lo, hi - lo);
+      }
+      __syncthreads();
+      below = A.tail_start[k];
+      cnt = np;
+    }
   }
 }
 
@@ -387,28 +487,52 @@ int build_tree(const float* in_xmin, const float* in_ymin, const float* in_xmax,
     CRT_LAUNCHED(1);
     sort_passes(cols, n, kDigits, scratch, stream);
 
-    // leaf-parent level
-    int64_t parent_start = rsz;
-    int64_t child_start = 0, nchild = n;
-    for (size_t l = 0; l < lv.size(); l++) {
-      const int64_t np = lv[l];
-      parent_start -= np;
-      int npc = (int)std::max<int64_t>(1, std::min<int64_t>(kLevelThreads, kLevelChunk / fanout));
-      unsigned g = (unsigned)cdiv(np, npc);
+    // the levels, leaf-parents first: start[l] is level l's first node
+    std::vector<int64_t> start(lv.size());
+    int64_t at = rsz;
+    for (size_t l = 0; l < lv.size(); l++) start[l] = at -= lv[l];
+    const NodeOut nodes{nxmin, nymin, nxmax, nymax, npos, nlen};
+    int launch = 0;
+    for (size_t l = 0; l < lv.size(); launch++) {
+      LevelArgs A{};
+      A.fanout = fanout;
+      A.nchild = l ? lv[l - 1] : n;
+      A.nparent = lv[l];
+      A.parent_start = (int)start[l];
+      A.child_start = l ? (int)start[l - 1] : 0;
+      A.pos_base = l ? A.child_start : (int)rsz;
+      // a launch of one wave goes on upwards: whole subtrees per CTA as far as
+      // its parents go.  In longer launches the extra steps (and the last CTA's
+      // fence) cost every wave more than the launches they save (10M boxes,
+      // fanout 16: leaf level 176 us with them, 165 without).
+      const int64_t most = std::max<int64_t>(1, std::min<int64_t>(kLevelThreads, kLevelChunk / fanout));
+      const bool fuse = cdiv(A.nparent, most) <= (int64_t)sms * 4;
+      int64_t sub = 1;
+      while (fuse && A.up_n < kUpMax && l + 1 + A.up_n < lv.size() && sub * fanout <= most) {
+        sub *= fanout;
+        A.up_start[A.up_n] = (int)start[l + 1 + A.up_n];
+        A.up_n++;
+      }
+      A.nodes_per_cta = (int)(most / sub * sub);
+      size_t top = l + A.up_n;  // the last level made so far
+      if (fuse && lv[top] <= kTailNodes && launch < (int)(sizeof(ctrl->level_done) / sizeof(int))) {
+        A.tail_child = (int)start[top];
+        A.tail_nchild = (int)lv[top];
+        while (A.tail_n < kTailMax && top + 1 < lv.size()) A.tail_start[A.tail_n++] = (int)start[++top];
+        A.done = &ctrl->level_done[launch];
+      }
+      const unsigned g = (unsigned)cdiv(A.nparent, A.nodes_per_cta);
       ProfScope ps("level", stream);
       if (l == 0)
-        level_kernel<true><<<g, kLevelThreads, 0, stream>>>(
-            npc, fanout, nchild, np, parent_start, rsz, cols.val[0], cols.val[1], ctrl, aos,
-            out_xmin, out_ymin, out_xmax, out_ymax, out_id, nxmin, nymin, nxmax, nymax, npos,
-            nlen, 0);
+        launch_after(fuse ? level_kernel<true, true> : level_kernel<true, false>, g, kLevelThreads, 0,
+                     stream, A, nodes, cols.val[0], cols.val[1], ctrl, aos, out_xmin, out_ymin, out_xmax,
+                     out_ymax, out_id);
       else
-        level_kernel<false><<<g, kLevelThreads, 0, stream>>>(
-            npc, fanout, nchild, np, parent_start, child_start, nullptr, nullptr, ctrl, nullptr,
-            nullptr, nullptr, nullptr, nullptr, nullptr, nxmin, nymin, nxmax, nymax, npos, nlen,
-            child_start);
+        launch_after(fuse ? level_kernel<false, true> : level_kernel<false, false>, g, kLevelThreads, 0,
+                     stream, A, nodes, nullptr, nullptr, ctrl, nullptr, nullptr, nullptr, nullptr,
+                     nullptr, nullptr);
       CRT_LAUNCHED(1);
-      child_start = parent_start;
-      nchild = np;
+      l = top + 1;
     }
     if (lv.empty()) {
       // one box, no nodes: the sorted box set is the input itself

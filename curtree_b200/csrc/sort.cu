@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   int* s_wsum = (int*)(sweep_smem + L::kWsum);
   __shared__ int s_tile, s_stop;
 
+  chain_wait();
   const int active = ctrl->active;
   if (!((active >> digit) & 1)) return;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     s_gbase[tid] = bucket + excl - binstart;
   }
   __syncthreads();
+  chain_next();
   if (s_stop) return;
 #pragma unroll
   for (int i = 0; i < kIpt; i++) {
@@ -270,10 +272,10 @@ struct SweepShape {
   int threads;
   int tile;
   size_t smem;
-  const void* fn;
+  void (*fn)(int, SortCols, int64_t, uint64_t*, SortCtrl*);
 };
 
-#define CRT_SHAPE(T, I, B) {T, (T) * (I), SweepSmem<T, I>::kBytes, (const void*)sweep_kernel<T, I, B>}
+#define CRT_SHAPE(T, I, B) {T, (T) * (I), SweepSmem<T, I>::kBytes, sweep_kernel<T, I, B>}
 // Tile shapes by pair count: {most pairs, shape}.  A tile's fixed cost (ticket,
 // bin scan, look-back) is a few microseconds whatever its size, so large sorts
 // want large tiles; small ones want enough tiles to use the SMs.  Sort of a
@@ -316,13 +318,15 @@ void sort_passes(const SortCols& cols, int64_t n, int digits, void* zero_block, 
   const SweepShape& S = shape_for(n);
   const int64_t tiles = sort_tiles(n);
   SortCtrl* ctrl = sort_ctrl(zero_block);
-  cudaFuncSetAttribute(S.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S.smem);
+  // a pass of at most one tile per SM asks for more than half of an SM's shared
+  // memory: started while the pass before drains, its CTAs would otherwise share
+  // the first SMs that fall free
+  const size_t smem = tiles <= sm_count() ? std::max<size_t>(S.smem, 116 * 1024) : S.smem;
+  cudaFuncSetAttribute(S.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   for (int d = 0; d < digits; d++) {
     ProfScope ps("sort_pass", stream);
     uint64_t* status = (uint64_t*)(ctrl + 1) + (size_t)d * tiles * kBins;
-    SortCols c = cols;
-    void* args[] = {&d, &c, &n, &status, &ctrl};
-    cudaLaunchKernel(S.fn, dim3((unsigned)tiles), dim3(S.threads), args, S.smem, stream);
+    launch_after(S.fn, (unsigned)tiles, S.threads, smem, stream, d, cols, n, status, ctrl);
   }
   CRT_LAUNCHED(digits);
 }

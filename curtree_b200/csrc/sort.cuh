@@ -23,7 +23,7 @@ struct SortCtrl {
   int active;                 // bit d: digit d is not uniform
   int n_active;               // number of active passes
   int done;                   // CTAs of the key kernel that have added their histograms
-  int pad[4];
+  int level_done[12];         // a build's level launches: CTAs finished
   uint32_t hist[2 * kDigits * kBins];     // digit histograms, filled by the key kernel
   int bucket_start[2 * kDigits * kBins];  // exclusive prefix of each digit's histogram
 };

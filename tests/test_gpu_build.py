@@ -146,3 +146,26 @@ def test_build_matches_reference_golden(crt, path):
         assert _bits_equal(getattr(h, k), z["node_" + k]), k
     assert np.array_equal(h.pos, z["node_pos"]) and np.array_equal(h.len, z["node_len"])
     rt.free()
+
+
+@pytest.mark.parametrize("fanout", [2, 3, 7, 10, 16, 45, 46, 100, 300, 2100])
+def test_levels_at_cta_and_tail_edges(crt, fanout):
+    """Node arrays at sizes where a level launch's shape changes: one box past
+    whole subtrees of a CTA, one CTA and several, levels of one node, and the
+    last CTA's part of the tree (at most 16384 children)."""
+    per = max(1, min(256, 2048 // fanout))
+    sub = 1
+    while sub * fanout <= per:
+        sub *= fanout
+    cta = per // sub * sub * fanout  # boxes of one leaf-level CTA
+    for n in sorted({2, fanout, fanout + 1, cta - 1, cta, cta + 1, 3 * cta + 1, fanout * fanout + 1,
+                     16384 * fanout + 1 if fanout < 20 else 2 * cta}):
+        b = D.uniform_boxes(n, seed=n % 1000)
+        d, rt = crt.build_into(crt.BBox.from_host(b), fanout)
+        sb, t = O.build(b, fanout)
+        h = rt.to_host()
+        assert rt.sz == t.sz, (n, fanout)
+        for f in ("xmin", "ymin", "xmax", "ymax"):
+            assert np.array_equal(getattr(h, f).view(np.uint32), getattr(t, f).view(np.uint32)), (n, fanout, f)
+        assert np.array_equal(h.pos, t.pos) and np.array_equal(h.len, t.len), (n, fanout)
+        assert np.array_equal(d.to_host().id, sb.id)
