@@ -33,7 +33,7 @@ int cuda_fail(cudaError_t e, const char* what)
 
 // Keep freed stream-ordered blocks in the device pool between calls, so the
 // scratch of repeated builds and queries does not go back to the driver.
-static void init_device()
+void init_device()
 {
   static std::mutex mu;
   static std::vector<int> done;

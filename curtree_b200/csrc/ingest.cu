@@ -44,6 +44,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -468,11 +469,17 @@ __global__ void __launch_bounds__(kParseThreads)
 // Host side
 // ---------------------------------------------------------------------------
 
-// Pinned staging slots, two per copy thread, allocated on first use and kept
-// for the life of the process.
+// Pinned staging slots, two per copy thread, and each device's copy streams and
+// events, one set per copy thread: made on first use and kept for the life of
+// the process (at most kStageThreads of each), used by one call at a time.
+struct StageLane {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t done[2] = {nullptr, nullptr};
+};
 struct StagePool {
   std::mutex mu;
   char* slot[kStageThreads][2] = {};
+  std::map<int, std::vector<StageLane>> lanes;  // by device
 };
 
 StagePool& stage_pool()
@@ -536,10 +543,12 @@ struct Source {
 // file instead of pread 14.8.
 int stage_text(char* d_text, Source& src, int dev)
 {
-  const int64_t nchunks = cdiv(src.len, (int64_t)kStageChunk);
-  if (nchunks == 0) return CRT_OK;
-  const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
-  const int nt = (int)std::min<int64_t>(std::min(kStageThreads, hw), nchunks);
+  if (src.len == 0) return CRT_OK;
+  const int hw = std::min(kStageThreads, (int)std::max(1u, std::thread::hardware_concurrency()));
+  const int64_t chunk =
+      std::min<int64_t>((int64_t)kStageChunk, std::max<int64_t>(256 << 10, cdiv(src.len, 2 * hw * 65536ll) * 65536));
+  const int64_t nchunks = cdiv(src.len, chunk);
+  const int nt = (int)std::min<int64_t>(hw, nchunks);
   StagePool& P = stage_pool();
   std::lock_guard<std::mutex> lock(P.mu);
   for (int t = 0; t < nt; t++)  // the slots of the threads this call uses
@@ -550,44 +559,70 @@ int stage_text(char* d_text, Source& src, int dev)
         P.slot[t][s] = nullptr;
         return fail(CRT_ERR_OOM, "read_mbr_csv_device: pinned staging allocation failed");
       }
+  std::vector<StageLane>& lanes = P.lanes[dev];
+  while ((int)lanes.size() < nt) {
+    StageLane l;
+    cudaError_t e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
+    for (int s = 0; s < 2 && e == cudaSuccess; s++)
+      e = cudaEventCreateWithFlags(&l.done[s], cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+      for (auto ev : l.done)
+        if (ev) cudaEventDestroy(ev);
+      if (l.stream) cudaStreamDestroy(l.stream);
+      return cuda_fail(e, "read_mbr_csv_device: staging stream");
+    }
+    lanes.push_back(l);
+  }
   std::vector<int> bad_read(nt, 0);
   std::vector<cudaError_t> err(nt, cudaSuccess);
+  auto copy = [&](int t) {
+    cudaError_t& e = err[t];
+    const StageLane& L = lanes[t];
+    e = cudaSetDevice(dev);
+    int it = 0;
+    for (int64_t c = t; c < nchunks && e == cudaSuccess && !bad_read[t]; c += nt, it++) {
+      const int s = it & 1;
+      if (it >= 2) e = cudaEventSynchronize(L.done[s]);  // the slot's previous copy is done
+      if (e != cudaSuccess) break;
+      const int64_t off = c * chunk;
+      const size_t m = (size_t)std::min<int64_t>(chunk, src.len - off);
+      if (src.mem) std::memcpy(P.slot[t][s], src.mem + off, m);
+      else if (!src.read_at(P.slot[t][s], off, m)) bad_read[t] = 1;
+      if (!bad_read[t])
+        e = cudaMemcpyAsync(d_text + off, P.slot[t][s], m, cudaMemcpyHostToDevice, L.stream);
+      if (!bad_read[t] && e == cudaSuccess) e = cudaEventRecord(L.done[s], L.stream);
+    }
+    const cudaError_t es = cudaStreamSynchronize(L.stream);
+    if (e == cudaSuccess) e = es;
+  };
   std::vector<std::thread> th;
-  for (int t = 0; t < nt; t++) {
-    th.emplace_back([&, t] {
-      cudaError_t& e = err[t];
-      e = cudaSetDevice(dev);
-      cudaStream_t st;
-      cudaEvent_t ev[2];
-      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-      if (e != cudaSuccess) return;
-      cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming);
-      cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming);
-      int it = 0;
-      for (int64_t c = t; c < nchunks && e == cudaSuccess && !bad_read[t]; c += nt, it++) {
-        const int s = it & 1;
-        if (it >= 2) e = cudaEventSynchronize(ev[s]);  // the slot's previous copy is done
-        if (e != cudaSuccess) break;
-        const int64_t off = c * (int64_t)kStageChunk;
-        const size_t m = (size_t)std::min<int64_t>((int64_t)kStageChunk, src.len - off);
-        if (src.mem) std::memcpy(P.slot[t][s], src.mem + off, m);
-        else if (!src.read_at(P.slot[t][s], off, m)) bad_read[t] = 1;
-        if (!bad_read[t]) e = cudaMemcpyAsync(d_text + off, P.slot[t][s], m, cudaMemcpyHostToDevice, st);
-        if (!bad_read[t] && e == cudaSuccess) e = cudaEventRecord(ev[s], st);
-      }
-      const cudaError_t es = cudaStreamSynchronize(st);
-      if (e == cudaSuccess) e = es;
-      cudaEventDestroy(ev[0]);
-      cudaEventDestroy(ev[1]);
-      cudaStreamDestroy(st);
-    });
-  }
+  for (int t = 1; t < nt; t++) th.emplace_back(copy, t);
+  copy(0);
   for (auto& x : th) x.join();
   for (int t = 0; t < nt; t++) {
     if (err[t] != cudaSuccess) return cuda_fail(err[t], "read_mbr_csv_device: staging copy");
     if (bad_read[t]) return fail(CRT_ERR_INVALID_ARG, "read_mbr_csv_device: reading the file failed");
   }
   return CRT_OK;
+}
+
+// Five box columns of m entries from the stream-ordered pool, which cudaFree
+// (the reference's box_d_free, src/utility.cuh:68-89) releases too: five
+// cudaMalloc calls took 2.4 of the 4.7 ms of reading a 26 MB text.  False, with
+// nothing allocated, when memory runs out.
+bool alloc_columns(void** const dst[5], int64_t m, cudaStream_t stream)
+{
+  for (int a = 0; a < 5 && m > 0; a++)
+    if (cudaMallocAsync(dst[a], (size_t)m * 4, stream) != cudaSuccess) {
+      cudaGetLastError();
+      *dst[a] = nullptr;
+      for (int b = 0; b < a; b++) {
+        cudaFreeAsync(*dst[b], stream);
+        *dst[b] = nullptr;
+      }
+      return false;
+    }
+  return true;
 }
 
 // Stream-ordered device allocations released when the call returns.
@@ -619,7 +654,7 @@ struct Outputs {
 };
 
 // The loader proper.  n < 0: every record (only when `alloc`).  alloc: the
-// outputs are cudaMalloc'd here for the records found (*box_out, freed on
+// outputs are allocated here for the records found (*box_out, freed on
 // failure); otherwise they are the caller's, of n entries.
 int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f32* box_out,
            int64_t* n_read, cudaStream_t stream)
@@ -627,6 +662,7 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
   if (n_read) *n_read = 0;
   int dev = 0;
   CRT_CUDA(cudaGetDevice(&dev));
+  init_device();
   const int64_t ntiles = cdiv(src.len, kLineTile);
   const size_t text_bytes = (size_t)ntiles * kLineTile + kTextPad;
   Scratch S(stream);
@@ -666,18 +702,14 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
     if (m > INT32_MAX) return fail(CRT_ERR_INVALID_ARG, "read_mbr_csv_device: more than 2^31-1 records");
     void** dst[5] = {(void**)&out.xmin, (void**)&out.ymin, (void**)&out.xmax, (void**)&out.ymax,
                      (void**)&out.id};
-    for (int a = 0; a < 5 && m > 0; a++)
-      if (cudaMalloc(dst[a], (size_t)m * 4) != cudaSuccess) {
-        cudaGetLastError();
-        for (int b = 0; b < a; b++) cudaFree(*dst[b]);
-        return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
-      }
+    if (!alloc_columns(dst, m, stream))
+      return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
   }
   auto release = [&] {
     if (alloc) {
       void* p[5] = {out.xmin, out.ymin, out.xmax, out.ymax, out.id};
       for (void* q : p)
-        if (q) cudaFree(q);
+        if (q) cudaFreeAsync(q, stream);
     }
   };
 
@@ -803,12 +835,9 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
           void** dst[5] = {(void**)&out.xmin, (void**)&out.ymin, (void**)&out.xmax,
                            (void**)&out.ymax, (void**)&out.id};
           for (int a2 = 0; a2 < 5; a2++) *dst[a2] = nullptr;
-          for (int a2 = 0; a2 < 5 && m > 0; a2++)
-            if (cudaMalloc(dst[a2], (size_t)m * 4) != cudaSuccess) {
-              cudaGetLastError();
-              for (int b2 = 0; b2 < a2; b2++) cudaFree(*dst[b2]);
-              return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
-            }
+          if (!alloc_columns(dst, m, stream))
+            return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
+          e = cudaStreamSynchronize(stream);  // the copies below run on another stream
         }
         const size_t bytes = (size_t)std::min<int64_t>(rec.count, m) * 4;
         float* dv[4] = {out.xmin, out.ymin, out.xmax, out.ymax};
@@ -888,6 +917,7 @@ int ingest_bin(Source& src, int64_t n, float r, crt_bbox_f32* box_out, int64_t* 
   if (m > 0) {
     int dev = 0;
     CRT_CUDA(cudaGetDevice(&dev));
+    init_device();
     Scratch S(stream);
     char* raw = S.get<char>((size_t)(m * kBinRecord) + 256);
     if (!raw) return fail(CRT_ERR_OOM, "read_mbr_bin_device: device allocation failed");
@@ -898,12 +928,8 @@ int ingest_bin(Source& src, int64_t n, float r, crt_bbox_f32* box_out, int64_t* 
     if (rc != CRT_OK) return rc;
     void** dst[5] = {(void**)&box.xmin, (void**)&box.ymin, (void**)&box.xmax, (void**)&box.ymax,
                      (void**)&box.id};
-    for (int a = 0; a < 5; a++)
-      if (cudaMalloc(dst[a], (size_t)m * 4) != cudaSuccess) {
-        cudaGetLastError();
-        for (int b = 0; b < a; b++) cudaFree(*dst[b]);
-        return fail(CRT_ERR_OOM, "read_mbr_bin_device: output allocation failed");
-      }
+    if (!alloc_columns(dst, m, stream))
+      return fail(CRT_ERR_OOM, "read_mbr_bin_device: output allocation failed");
     const int64_t grid = std::min<int64_t>(cdiv(m, kParseThreads), (int64_t)sm_count() * 16);
     mbr_bin_kernel<<<(unsigned)grid, kParseThreads, 0, stream>>>(
         (const uint32_t*)d_rec, m, r, box.xmin, box.ymin, box.xmax, box.ymax, box.id);

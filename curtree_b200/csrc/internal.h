@@ -11,6 +11,9 @@
 
 namespace crt {
 
+// Once per device: the stream-ordered pool keeps what is freed.
+void init_device();
+
 int tree_levels(int64_t n, int fanout, std::vector<int64_t>& lv);
 
 int build_tree(const float* in_xmin, const float* in_ymin, const float* in_xmax,

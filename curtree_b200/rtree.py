@@ -61,10 +61,10 @@ def _d2h(ptr: int, n: int, dtype) -> np.ndarray:
 
 
 def _copy_ptr(dst: int, src: int, nbytes: int) -> None:
-    """Device-to-device copy between raw addresses on the current stream."""
+    """Device-to-device copy between raw addresses on the current stream
+    (asynchronous)."""
     if nbytes:
         _device_bytes(dst, nbytes).copy_(_device_bytes(src, nbytes))
-        torch.cuda.current_stream().synchronize()
 
 
 class BBox:
@@ -460,6 +460,7 @@ def _read_mbr(fn: str, path, n: int, r: float, stream) -> BBox:
             for dst, src in ((out.xmin, box.xmin), (out.ymin, box.ymin), (out.xmax, box.xmax),
                              (out.ymax, box.ymax), (out.id, box.id)):
                 _copy_ptr(dst.data_ptr(), src, 4 * int(box.sz))
+            torch.cuda.current_stream().synchronize()  # before the library's arrays are freed
     finally:
         L.crt_bbox_free(ctypes.byref(box))
     return out
