@@ -74,6 +74,7 @@ struct Hole {
 // ---------------------------------------------------------------------------
 struct CountEmit {
   static constexpr bool kCountsTests = false;
+  static constexpr int kSmall = kSmallRange;
   long long hits = 0;
   __device__ __forceinline__ void begin(int) {}
   __device__ __forceinline__ void operator()(bool hit, int) { hits += __popc(__ballot_sync(0xffffffffu, hit)); }
@@ -91,6 +92,7 @@ struct CountEmit {
 // Counts hits and the leaf boxes tested (workload statistics).
 struct StatEmit {
   static constexpr bool kCountsTests = true;
+  static constexpr int kSmall = kSmallRange;
   long long hits = 0;
   long long tested = 0;
   __device__ __forceinline__ void begin(int) {}
@@ -117,6 +119,7 @@ struct StatEmit {
 // Writes at precomputed per-window offsets (plain write pass).
 struct OffsetEmit {
   static constexpr bool kCountsTests = false;
+  static constexpr int kSmall = kSmallRange;
   int32_t* fid;
   int32_t* tid;
   long long base;
@@ -226,6 +229,8 @@ __device__ __forceinline__ int wait_piece(JobQueue* Q, const QueryCounters* ctr,
 // Warp-reserved output chunks (persistent form).
 struct ChunkEmit {
   static constexpr bool kCountsTests = false;
+  // runs of 64 boxes and more are queued (32: the same, 128: 2% slower, 256: 6%)
+  static constexpr int kSmall = 64;
   int32_t* fid;
   int32_t* tid;
   long long cap;
@@ -263,36 +268,58 @@ struct ChunkEmit {
   }
   __device__ __forceinline__ void small_ranges(const int* bid, bool mine, long long first, int count)
   {
+    if (cur >= cap && cur < end) {  // past the output: only the count matters
+      hits += __reduce_add_sync(0xffffffffu, mine ? (unsigned)count : 0u);
+      return;
+    }
     emit_small_ranges(*this, bid, mine, first, count);
   }
-  // Large contained subtrees go to an exact reservation (no unused chunk
-  // end), all of one step's in one: each lane's range at its prefix offset.
-  // One atomic per step instead of one per range keeps the shared output
-  // counter from becoming the bottleneck when every warp meets large
-  // subtrees at once (10M boxes x 250k windows of side 1e-2..1e-1: 21 ms
-  // with one atomic per range, 12.4 ms with one per step).
+  // Large contained runs go to exact reservations (no unused chunk end), 32 of
+  // them in one: the warp queues them and reserves for all when 32 wait, or when
+  // its window ends.  Every warp reserves from one counter, and that counter
+  // takes about one atomic per 1.6 ns: with one per range 10M boxes x 250k
+  // windows of side 1e-2..1e-1 took 21 ms, with one per step 12.4 (and 1M
+  // mixed windows 17.0 ms where runs down to 64 boxes came here, 11.2 queued).
+  int2* queue = nullptr;  // 64 entries of this warp: first slot, count
+  int queued = 0;
   __device__ __forceinline__ void big_ranges(const int* bid, bool mine, long long first, long long count)
   {
+    const uint32_t m = __ballot_sync(0xffffffffu, mine);
+    if (mine) queue[queued + __popc(m & lanemask_lt())] = make_int2((int)first, (int)count);
+    queued += __popc(m);
+    __syncwarp();
+    if (queued >= 32) {
+      flush_ranges(bid);
+      // the entries past the first 32 move down
+      const int lane = (int)lane_id();
+      int2 rest = make_int2(0, 0);
+      if (lane < queued) rest = queue[32 + lane];
+      __syncwarp();
+      if (lane < queued) queue[lane] = rest;
+      __syncwarp();
+    }
+  }
+  // Places the first 32 queued ranges (all, when there are fewer).
+  __device__ __forceinline__ void flush_ranges(const int* bid)
+  {
     const int lane = (int)lane_id();
-    const long long c = mine ? count : 0;
-    long long x = c;
+    const int n = min(queued, 32);
+    if (n == 0) return;
+    const int2 r = lane < n ? queue[lane] : make_int2(0, 0);
+    long long x = r.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const long long y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    const long long total = __shfl_sync(0xffffffffu, x, 31);
     unsigned long long nb = 0;
-    if (lane == 0) nb = atomicAdd(next, (unsigned long long)total);
-    nb = __shfl_sync(0xffffffffu, nb, 0);
-    const long long excl = x - c;
-    uint32_t im = __ballot_sync(0xffffffffu, mine);
-    while (im) {
-      const int src = __ffs(im) - 1;
-      im &= im - 1;
-      place(bid, __shfl_sync(0xffffffffu, first, src), __shfl_sync(0xffffffffu, count, src),
-            (long long)nb + __shfl_sync(0xffffffffu, excl, src));
-    }
+    if (lane == 31) nb = atomicAdd(next, (unsigned long long)x);
+    nb = __shfl_sync(0xffffffffu, nb, 31);
+    const long long excl = x - r.y;
+    for (int i = 0; i < n; i++)
+      place(bid, __shfl_sync(0xffffffffu, r.x, i), __shfl_sync(0xffffffffu, r.y, i),
+            (long long)nb + __shfl_sync(0xffffffffu, excl, i));
+    queued -= n;
   }
   // Copies a contained subtree's ids to its reservation at output slot nb
   // (large ones cut into pieces that idle warps copy).
@@ -300,6 +327,7 @@ struct ChunkEmit {
                                         long long nb)
   {
     hits += count;
+    if (nb >= cap) return;  // past the output: only the count matters
     if (!jobs || count < kShareMin) {
       copy_range_realign(bid, first, count, fid, tid, nb, cap, q);
       return;
@@ -548,7 +576,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   __shared__ int s_stage_ok;
   const int warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
-  // layout: [staged nodes: 6 arrays x stage_n x 4 B][stacks: warps x stack_cap x 4 B]
+  // layout: [staged nodes: 6 arrays x stage_n x 4 B][stacks: warps x stack_cap
+  // entries][queued ranges: warps x 64]
   float* c_xmin = (float*)smem_raw;
   float* c_ymin = c_xmin + P.stage_n;
   float* c_xmax = c_ymin + P.stage_n;
@@ -600,6 +629,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 
   FrontierEntry* stack = stacks + warp * P.stack_cap;
+  int2* queue = (int2*)(stacks + warps * P.stack_cap) + warp * 64;
   int lg, lc;
   lane_map(P.T.fanout, lg, lc);
   const uint32_t* order = nullptr;
@@ -620,6 +650,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   emit.cap = P.cap;
   emit.next = &P.ctr->next;
   emit.chunk = P.chunk;
+  emit.queue = queue;
   emit.jobs = kShare ? P.jobs : nullptr;
   JobQueue* Q = kShare ? P.jobs : nullptr;
   // a warp counts as active from before its first ticket until it has left
@@ -656,6 +687,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     emit.begin(q);
     traverse(P.T, C, P.K, lg, lc, P.W.xmin[q], P.W.ymin[q], P.W.xmax[q], P.W.ymax[q], stack,
              P.stack_cap, emit, &P.ctr->error, part, nparts, split);
+    emit.flush_ranges(P.T.bid);
   }
   if (Q) {
     __syncwarp();
@@ -725,6 +757,7 @@ constexpr int kPairChunk = 32;  // frontier nodes whose pairs are listed at a ti
 
 struct StageEmit {
   static constexpr bool kCountsTests = false;
+  static constexpr int kSmall = kSmallRange;
   int2* s_out;  // this warp's staging, kSmallStage pairs
   int n = 0;
   int q = 0;  // the window, where the warp walks one at a time
@@ -1485,7 +1518,7 @@ static PersistShape persist_shape(int stack_cap, int stage_n, int warps_per_cta)
   const size_t per_sm = 227 * 1024;
   for (int pass = 0; pass < 3; pass++) {
     const int sn = pass == 0 ? stage_n : 0;
-    const size_t smem = (size_t)sn * 24 + (size_t)(v.threads / 32) * stack_cap * sizeof(FrontierEntry);
+    const size_t smem = (size_t)sn * 24 + (size_t)(v.threads / 32) * (stack_cap + 64) * sizeof(FrontierEntry);
     const size_t limit = pass < 2 ? per_sm / v.min_blocks - 1024 : 220 * 1024;
     if (smem <= limit) return PersistShape{&v, sn, smem};
   }

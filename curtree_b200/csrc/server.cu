@@ -122,6 +122,7 @@ __device__ __forceinline__ unsigned long long ld_volatile_u64(const unsigned lon
 
 struct StagedEmit {
   static constexpr bool kCountsTests = false;
+  static constexpr int kSmall = kSmallRange;
   int32_t* s_fid;  // this warp's staging, kStage entries
   int32_t* s_tid;
   int n = 0;
