@@ -43,19 +43,25 @@ inline int sm_count()
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Programmatic dependent launch along a stream: a kernel launched with
-// launch_after may start while the one before it drains, and waits in
-// chain_wait() for that one to complete (its writes are then visible).  Every
-// thread of such a kernel calls chain_wait() before it touches memory, also
-// where it leaves at once, so that its completion implies the completion of
-// everything before it.  It hides the launch latency between the short kernels
-// of a load or a sort (canonical order of 384k pairs: 102 us without, 85 with;
-// 10.8M: 535, 502).  A kernel lets the next one start (chain_next) only before
-// its last stores: started at once, the next kernel's CTAs crowd onto the SMs
-// that fall free first (10M-box build 671 us against 711).  While a stream is
-// captured into a graph the launch is an ordinary one.
+// launch_after or launch_beside may start while the one before it still runs,
+// as soon as every CTA of that one has called chain_next() or left.
+//
+// launch_after: for a kernel that needs the one before it.  Every thread calls
+// chain_wait() before it touches memory, also where it leaves at once: it waits
+// for the kernel before to complete (its writes are then visible), so that its
+// own completion implies the completion of everything before it.  It hides the
+// launch latency between the short kernels of a load or a sort (canonical order
+// of 384k pairs: 102 us without, 85 with; 10.8M: 535, 502).  A kernel lets the
+// next one start only before its last stores: started at once, the next
+// kernel's CTAs crowd onto the SMs that fall free first (10M-box build 671 us
+// against 711).  While a stream is captured into a graph the launch is an
+// ordinary one.
+//
+// launch_beside: for a kernel that needs only what lies before the one before
+// it; it calls chain_wait() last.
 template <class... P, class... A>
-inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
-                                cudaStream_t stream, A... args)
+inline cudaError_t launch_chained(bool early, void (*kernel)(P...), unsigned grid, unsigned threads,
+                                  size_t smem, cudaStream_t stream, A... args)
 {
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
@@ -63,14 +69,25 @@ inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned th
   c.dynamicSmemBytes = smem;
   c.stream = stream;
   cudaLaunchAttribute a{};
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    a.val.programmaticStreamSerializationAllowed = 1;
-    c.attrs = &a;
-    c.numAttrs = 1;
-  }
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &a;
+  c.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_after(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                                cudaStream_t stream, A... args)
+{
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool live = cudaStreamIsCapturing(stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  return launch_chained(live, kernel, grid, threads, smem, stream, args...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_beside(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                                 cudaStream_t stream, A... args)
+{
+  return launch_chained(true, kernel, grid, threads, smem, stream, args...);
 }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the next kernel of the chain start (it waits for this one's end).
