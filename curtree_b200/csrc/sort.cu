@@ -4,15 +4,15 @@
 // the passes (sort_plan, sort.cuh); every pass then is one launch that reads
 // and writes the pairs once, with decoupled look-back across tiles.
 //
-// A pass is bound by instruction issue (the in-warp ranking) and by the chain
-// ticket -> keys -> ranks -> bin scan -> look-back -> stores inside a tile,
-// not by DRAM: 100M pairs take 0.58 ms per pass, 2.8 TB/s.  What shortened the
+// A pass is bound by instruction issue, the shared-memory pipe and the chain
+// ticket -> keys -> ranks -> bin scan -> look-back -> stores inside a tile, not
+// by DRAM: 100M pairs take 0.56 ms per pass, 2.9 TB/s.  What shortened the
 // chain (0.67 ms before): the values go through registers, on their way while
 // the bins are scanned, instead of through a third shared-memory buffer; the
 // look-back comes after the staging, when the predecessors have mostly
 // published; no second launch to plan the passes.  CTAs that stay resident
 // and fetch their next tile's ticket and keys early measured slower (2.94
-// against 2.30 ms): a claimed tile waits for its CTA, and every successor's
+// against 2.30 ms then): a claimed tile waits for its CTA, and every successor's
 // look-back waits for that tile.
 #include <cuda_runtime.h>
 
@@ -275,25 +275,23 @@ struct SweepShape {
 #define CRT_SHAPE(T, I, B) {T, (T) * (I), SweepSmem<T, I>::kBytes, sweep_kernel<T, I, B>}
 // Tile shapes by pair count: {most pairs, shape}.  A tile's fixed cost (ticket,
 // bin scan, look-back) is a few microseconds whatever its size, so large sorts
-// want large tiles; small ones want enough tiles to use the SMs.  Sort of a
-// build (four passes, us with event overhead), by tile size:
-//   pairs   1024   4096   6144   8192
-//    20k      39     48     50     54
-//   200k      52     51     59     59
-//     1M     103     70     75     66
-//     3M     239    135    123    139
-//    10M     704    323    290    292
-//   100M    6717   2624   2361   2300
-// (1M: one tile of 8192 per SM, a single wave.)
+// want large tiles, as large as the registers hold without spills (512 threads
+// x 14; x 16 spills); small ones want enough tiles to use the SMs.  Sort of a
+// build (four passes, us with event overhead), by threads x keys:
+//   pairs   256x4  256x8  256x16  384x16  512x14  512x16  512x20
+//    20k       37     43      43      49      49      52      57
+//   200k       49     45      50      51      52      58      59
+//     1M        -     73      67      65      59      64      65
+//     3M        -    133     123     110     112     112     100
+//    10M        -    346     291     270     260     272     274
+//   100M        -   3192    2619    2394    2241    2279    2369
 static const struct {
   int64_t most;
   SweepShape shape;
 } kShapes[] = {
     {1 << 16, CRT_SHAPE(256, 4, 4)},
-    {3 << 18, CRT_SHAPE(256, 16, 4)},
-    {148 * 8192, CRT_SHAPE(512, 16, 2)},
-    {10'000'000, CRT_SHAPE(384, 16, 3)},
-    {INT64_MAX, CRT_SHAPE(512, 16, 2)},
+    {400'000, CRT_SHAPE(256, 8, 6)},
+    {INT64_MAX, CRT_SHAPE(512, 14, 2)},
 };
 
 static const SweepShape& shape_for(int64_t n)
