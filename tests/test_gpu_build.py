@@ -169,3 +169,23 @@ def test_levels_at_cta_and_tail_edges(crt, fanout):
             assert np.array_equal(getattr(h, f).view(np.uint32), getattr(t, f).view(np.uint32)), (n, fanout, f)
         assert np.array_equal(h.pos, t.pos) and np.array_equal(h.len, t.len), (n, fanout)
         assert np.array_equal(d.to_host().id, sb.id)
+
+
+@pytest.mark.parametrize("kind,n", [("uniform", (1 << 22) - 1), ("uniform", 1 << 22),
+                                    ("clustered", (1 << 22) + 4097), ("one_corner", 4_200_001)])
+def test_build_where_records_move_to_blocks(crt, kind, n):
+    """Around the size from which a top byte's records fill blocks of their own:
+    every top byte in use, few of them, and one that fills block after block."""
+    if kind == "clustered":
+        b = D.clustered_boxes(n, seed=5, chunk=n)
+    else:
+        b = D.uniform_boxes(n, seed=6)
+        if kind == "one_corner":  # all but one box in one top byte
+            s = np.float32(1 / 1024)
+            cols = [(a * s).astype(np.float32) for a in (b.xmin, b.ymin, b.xmax, b.ymax)]
+            for a, full in zip(cols, (b.xmin, b.ymin, b.xmax, b.ymax)):
+                a[n // 2] = full.max()
+            b = HostBoxes(*cols, b.id)
+    d, rt, rsz = gpu_build(crt, b, 10)
+    assert_tree_equal(crt, b, 10, d, rt, rsz)
+    rt.free()
