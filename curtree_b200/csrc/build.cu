@@ -62,7 +62,7 @@ static_assert(kGroups <= kEncThreads, "one thread per run");
 // translation (finer grouping inside the tile changes nothing).  100 M clustered
 // boxes: levels 2158 -> 1612 us for 80 us more in the encoder (the wait for the
 // run's place and shorter runs), build 5.65 -> 5.16 ms; 10 M: levels 177 -> 154,
-// encoder +7, build 655 -> 616 us; 3 M and fewer: no difference.
+// encoder +7, build 626 -> 613 us.
 struct BlockTable {
   uint32_t* cursor;  // per top byte: records placed so far (zeroed)
   uint32_t* block;   // per top byte and its k-th block: number + 1, 0 = none yet (zeroed)
@@ -491,10 +491,10 @@ int tree_levels(int64_t n, int fanout, std::vector<int64_t>& lv)
 
 static bool aligned16(const void* p) { return ((uintptr_t)p & 15u) == 0; }
 
-// Sets of at least this many boxes keep their records in blocks: below, the
-// copy (32 bytes a box) and the leaf level's outputs stay in the L2 and the
-// levels take the same time either way (3 M boxes: 64 us).
-constexpr int64_t kBlocksMin = 1 << 22;
+// Sets of at least this many boxes keep their records in blocks.  Build in
+// blocks against the tiles' own slots: 4.2 M boxes 328 to 320 us, 5 M 374 to
+// 368, 10 M 602 to 611 (uniform) and 613 to 626 (clustered).
+constexpr int64_t kBlocksMin = 1 << 23;
 // Records per block: the largest power of two up to 2^16 with at least
 // kBlockShare of them in the set, so the part-filled blocks (one per top byte)
 // add at most half to the copy.  10 M boxes: 2^14 154 us of levels, 2^13 162,

@@ -171,8 +171,8 @@ def test_levels_at_cta_and_tail_edges(crt, fanout):
         assert np.array_equal(d.to_host().id, sb.id)
 
 
-@pytest.mark.parametrize("kind,n", [("uniform", (1 << 22) - 1), ("uniform", 1 << 22),
-                                    ("clustered", (1 << 22) + 4097), ("one_corner", 4_200_001)])
+@pytest.mark.parametrize("kind,n", [("uniform", (1 << 23) - 1), ("uniform", 1 << 23),
+                                    ("clustered", (1 << 23) + 4097), ("one_corner", 8_400_001)])
 def test_build_where_records_move_to_blocks(crt, kind, n):
     """Around the size from which a top byte's records fill blocks of their own:
     every top byte in use, few of them, and one that fills block after block."""
