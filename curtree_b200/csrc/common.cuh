@@ -40,6 +40,22 @@ inline int sm_count()
   return n;
 }
 
+// Lets `fn` be launched with `smem` bytes of dynamic shared memory.  The limit
+// belongs to the function, not to the launch, so callers on other threads with
+// other sizes must not lower it between this call and the launch: up to
+// kSmemAsk they all set the same one.
+constexpr size_t kSmemAsk = 200 * 1024;
+inline void allow_smem(const void* fn, size_t smem)
+{
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)(smem > kSmemAsk ? smem : kSmemAsk));
+}
+template <typename... Args>
+inline void allow_smem(void (*fn)(Args...), size_t smem)
+{
+  allow_smem((const void*)fn, smem);
+}
+
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Programmatic dependent launch along a stream: a kernel launched with

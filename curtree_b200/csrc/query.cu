@@ -1498,7 +1498,7 @@ static const PersistVariant& variant_for(int warps_per_cta)
 static int persistent_grid(const PersistVariant& v, size_t smem)
 {
   int per_sm = 0;
-  cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(v.fn, smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.fn, v.threads, smem);
   if (per_sm < 1) per_sm = 1;
   return per_sm * sm_count();
@@ -1677,7 +1677,7 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
     L.small_warp_bytes = (int)SmallSmem::bytes(L.small.stack_cap);
     const size_t smem = (size_t)L.small_warp_bytes * kSmallWarps;
     int per_sm = 0;
-    cudaFuncSetAttribute(small_windows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(small_windows_kernel, smem);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, small_windows_kernel, kSmallWarps * 32, smem);
     L.small_grid = std::max(per_sm, 1) * sm_count();
   }
@@ -1790,7 +1790,7 @@ int query_dense(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   const bool few = T.nlev > 1 && W.n * kDenseParts <= (int64_t)sm_count() * kPlainWarps * 4;
   const int parts = few ? kDenseParts : 1;
   const size_t smem = dense_smem(sh.stack_cap);
-  cudaFuncSetAttribute(dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(dense_kernel, smem);
   {
     ProfScope ps("traverse_dense", stream);
     dense_kernel<<<(unsigned)cdiv(W.n * parts, kPlainWarps), kPlainWarps * 32, smem, stream>>>(
@@ -1836,8 +1836,8 @@ static void enqueue_plain(TreeView T, const LevelTables& lt, const WindowView& W
   cudaMemsetAsync(S.head, 0, plain_zero_bytes(nq), stream);
   attach_levels(T, lt, S.head + kHeadTables, nullptr, 0, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-  cudaFuncSetAttribute(plain_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(plain_write_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(plain_count_kernel, smem);
+  allow_smem(plain_write_kernel, smem);
   const unsigned g = (unsigned)cdiv(nq, kPlainWarps);
   if (nq > 0) {
     ProfScope ps("traverse_plain", stream);
@@ -2020,8 +2020,8 @@ int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   unsigned long long* tot = (unsigned long long*)(scr + 256);  // [3] box-by-box, [3] containment
   cudaMemsetAsync(scr, 0, 1024 + kLevelTableBytes, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-  cudaFuncSetAttribute(stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaFuncSetAttribute(stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem(stats_kernel<false>, smem);
+  allow_smem(stats_kernel<true>, smem);
   if (qbox.sz > 0) {
     const unsigned g = (unsigned)cdiv(qbox.sz, kPlainWarps);
     // the reference algorithm: every leaf box under an intersecting node is tested

@@ -189,3 +189,33 @@ def test_build_where_records_move_to_blocks(crt, kind, n):
     d, rt, rsz = gpu_build(crt, b, 10)
     assert_tree_equal(crt, b, 10, d, rt, rsz)
     rt.free()
+
+
+def test_builds_of_two_sizes_on_two_threads(crt):
+    """Two host threads build sets whose sort passes ask for different amounts
+    of shared memory: neither makes the other's launches fail."""
+    import threading
+
+    import torch
+    sets = [D.uniform_boxes(500_000, seed=7), D.uniform_boxes(1_500_000, seed=8)]
+    want = [O.build(b, 10)[0].id for b in sets]
+    bad = []
+
+    def run(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                d_in = crt.BBox.from_host(sets[k])
+                for _ in range(40):
+                    out, _ = crt.build_into(d_in, 10)
+                    got = out.id.cpu().numpy()
+                if not np.array_equal(got, want[k]):
+                    bad.append((k, "order differs"))
+        except Exception as e:  # noqa: BLE001 - reported by the main thread
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
