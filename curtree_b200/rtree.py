@@ -8,8 +8,8 @@ The names, argument meaning and ownership follow trxcllnt/curtree:
 with the reference's failure modes turned into exceptions (CrtError) instead
 of exit()/assert.  Device memory for inputs is allocated through PyTorch
 (plumbing only); node arrays and pair arrays returned by build/query are
-allocated by the library with cudaMalloc, exactly as the reference's
-rt_d_alloc / idpair_d_alloc do, and are released with free().
+allocated by the library from the device's stream-ordered pool in place of
+the reference's rt_d_alloc / idpair_d_alloc, and are released with free().
 
 Extended API: query_into (caller-owned output, int64 counts,
 overflow-and-retry, plain or persistent form) and Plan (a persistent query
@@ -100,7 +100,7 @@ class BBox:
 
 class RTree:
     """Node arrays in RTREE<float> layout.  `owned` trees were allocated by
-    build_rtree (library cudaMalloc) and are released by free(); trees built
+    build_rtree (the library's pool) and are released by free(); trees built
     with build_into wrap torch tensors."""
 
     def __init__(self, fanout: int):

@@ -385,11 +385,12 @@ int crt_server_destroy(crt_server s);
 /* ---------------------------------------------------------------------- */
 
 /* When enabled, the library brackets each major kernel launch (encode,
- * onesweep passes, level reductions, query traversal kernels, graph replays)
+ * sort passes, level reductions, query traversal kernels, graph replays)
  * with CUDA events on its own stream.  crt_profile_collect waits for them and
  * sums the durations of the launches named `name` (all when NULL/empty):
- * "encode", "sort_pass", "level", "traverse_persistent", "traverse_plain",
- * "plan". */
+ * "encode", "sort_pass", "level", "traverse_persistent" (with the small
+ * windows' kernel), "traverse_plain", "traverse_dense" (drop-in queries of
+ * small batches), "plan". */
 void crt_profile_enable(int on);
 int crt_profile_collect(const char* name, double* total_ms, int64_t* launches);
 
