@@ -4,7 +4,8 @@
 //   1. encode      read the box SoA (float4 loads where aligned), write the
 //                  flipped 32-bit Morton key and the slot of a 32-byte AoS
 //                  record of each box (records of a 4096-box tile grouped by
-//                  the key's top digit), and count all four 8-bit key digits.
+//                  the key's top byte, in large sets in blocks per top byte),
+//                  and count all four 8-bit key digits.
 //   2. plan        the encoder's last CTA: which digit passes are non-uniform (a
 //                  uniform digit leaves a stable order unchanged, so its pass is
 //                  skipped) and the global bucket start of every digit value.
@@ -40,7 +41,8 @@ struct alignas(32) Box32 {
 // ---------------------------------------------------------------------------
 // Each CTA takes tiles of kEncTile boxes.  Per box it writes the key and, in
 // input order, the slot of the box's 32-byte record; the records of a tile
-// are placed in its own slot range grouped by the key's top digit.  The sort
+// are placed in its own slot range (in large sets in blocks, below) grouped by
+// the key's top digit.  The sort
 // then carries those slots (its first pass reads them instead of making
 // input indices), and the leaf level's gather in sorted order, which walks
 // one top digit at a time, reads each tile's run for that digit (about
@@ -325,10 +327,11 @@ __device__ __forceinline__ float4 merge_box(float4 a, float4 m)
 // MBR, first child index, child count).  kLeaf: children are the sorted boxes,
 // gathered from the AoS copy through the sorted slot order, and the permuted
 // SoA is written on the way; otherwise children are nodes at child_start.
-// The leaf level is bound by its gathers: 100M clustered boxes take 2.1 ms, and
-// 0.86 with the records read in order; within windows of 32 MB (they fit the
-// L2 and few TLB entries) the same gathers take 1.2 ms.  Tile shapes, records
-// per thread in flight and 32-byte loads measured no difference.  A level above
+// The leaf level is bound by its gathers: 100M clustered boxes take 1.53 ms with
+// the records in blocks (2.1 in the tiles' own slots), 0.64 of the copy
+// bandwidth for its 64 bytes a box, and 0.86 with the records read in order.
+// Tile shapes, records per thread in flight and 32-byte loads measured no
+// difference.  A level above
 // it is a few microseconds of launch and latency, so a CTA goes on upwards over
 // the parents it holds in shared memory, and the last CTA makes the top of the
 // tree: one or two launches instead of one per level (all levels of 20k boxes,
