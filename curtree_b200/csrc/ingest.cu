@@ -606,22 +606,31 @@ int stage_text(char* d_text, Source& src, int dev)
   return CRT_OK;
 }
 
-// Five box columns of m entries from the stream-ordered pool, which cudaFree
-// (the reference's box_d_free, src/utility.cuh:68-89) releases too: five
-// cudaMalloc calls took 2.4 of the 4.7 ms of reading a 26 MB text.  False, with
-// nothing allocated, when memory runs out.
-bool alloc_columns(void** const dst[5], int64_t m, cudaStream_t stream)
+// Where a loader's five box columns come from.  kOwn: five cudaMalloc
+// allocations, as the C entry points promise them: cudaFree of one waits for
+// the work that still uses it, and they can be shared with other processes and
+// devices.  kPool: the stream-ordered pool, for a caller that copies the columns
+// away and waits for that before it frees them (the Python loaders): the five
+// cudaMalloc calls take 2.4 of the 4.7 ms of reading a 26 MB text.
+enum class Columns { kCallers, kOwn, kPool };
+
+// m entries per column.  False, with nothing allocated, when memory runs out.
+bool alloc_columns(Columns from, void** const dst[5], int64_t m, cudaStream_t stream)
 {
-  for (int a = 0; a < 5 && m > 0; a++)
-    if (cudaMallocAsync(dst[a], (size_t)m * 4, stream) != cudaSuccess) {
+  for (int a = 0; a < 5 && m > 0; a++) {
+    const size_t bytes = (size_t)m * 4;
+    const cudaError_t e = from == Columns::kPool ? cudaMallocAsync(dst[a], bytes, stream) : cudaMalloc(dst[a], bytes);
+    if (e != cudaSuccess) {
       cudaGetLastError();
       *dst[a] = nullptr;
       for (int b = 0; b < a; b++) {
-        cudaFreeAsync(*dst[b], stream);
+        if (from == Columns::kPool) cudaFreeAsync(*dst[b], stream);
+        else cudaFree(*dst[b]);
         *dst[b] = nullptr;
       }
       return false;
     }
+  }
   return true;
 }
 
@@ -653,12 +662,13 @@ struct Outputs {
   int32_t* id = nullptr;
 };
 
-// The loader proper.  n < 0: every record (only when `alloc`).  alloc: the
-// outputs are allocated here for the records found (*box_out, freed on
-// failure); otherwise they are the caller's, of n entries.
-int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f32* box_out,
+// The loader proper.  n < 0: every record (not into the caller's columns).  from:
+// the outputs are allocated there for the records found (*box_out, freed on
+// failure), or they are the caller's, of n entries.
+int ingest(Source& src, int64_t n, float r, Columns from, Outputs out, crt_bbox_f32* box_out,
            int64_t* n_read, cudaStream_t stream)
 {
+  const bool alloc = from != Columns::kCallers;
   if (n_read) *n_read = 0;
   int dev = 0;
   CRT_CUDA(cudaGetDevice(&dev));
@@ -702,14 +712,17 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
     if (m > INT32_MAX) return fail(CRT_ERR_INVALID_ARG, "read_mbr_csv_device: more than 2^31-1 records");
     void** dst[5] = {(void**)&out.xmin, (void**)&out.ymin, (void**)&out.xmax, (void**)&out.ymax,
                      (void**)&out.id};
-    if (!alloc_columns(dst, m, stream))
+    if (!alloc_columns(from, dst, m, stream))
       return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
   }
   auto release = [&] {
     if (alloc) {
       void* p[5] = {out.xmin, out.ymin, out.xmax, out.ymax, out.id};
-      for (void* q : p)
-        if (q) cudaFreeAsync(q, stream);
+      for (void* q : p) {
+        if (!q) continue;
+        if (from == Columns::kPool) cudaFreeAsync(q, stream);
+        else cudaFree(q);
+      }
     }
   };
 
@@ -835,7 +848,7 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
           void** dst[5] = {(void**)&out.xmin, (void**)&out.ymin, (void**)&out.xmax,
                            (void**)&out.ymax, (void**)&out.id};
           for (int a2 = 0; a2 < 5; a2++) *dst[a2] = nullptr;
-          if (!alloc_columns(dst, m, stream))
+          if (!alloc_columns(from, dst, m, stream))
             return fail(CRT_ERR_OOM, "read_mbr_csv_device: output allocation failed");
           e = cudaStreamSynchronize(stream);  // the copies below run on another stream
         }
@@ -897,8 +910,8 @@ int ingest(Source& src, int64_t n, float r, bool alloc, Outputs out, crt_bbox_f3
 
 // The binary loader: the first m records of the file staged to the device
 // like the text, then one thread per record.
-int ingest_bin(Source& src, int64_t n, float r, crt_bbox_f32* box_out, int64_t* n_read,
-               cudaStream_t stream)
+int ingest_bin(Source& src, int64_t n, float r, Columns from, crt_bbox_f32* box_out,
+               int64_t* n_read, cudaStream_t stream)
 {
   if (n_read) *n_read = 0;
   if (src.len % kBinRecord)
@@ -928,7 +941,7 @@ int ingest_bin(Source& src, int64_t n, float r, crt_bbox_f32* box_out, int64_t* 
     if (rc != CRT_OK) return rc;
     void** dst[5] = {(void**)&box.xmin, (void**)&box.ymin, (void**)&box.xmax, (void**)&box.ymax,
                      (void**)&box.id};
-    if (!alloc_columns(dst, m, stream))
+    if (!alloc_columns(from, dst, m, stream))
       return fail(CRT_ERR_OOM, "read_mbr_bin_device: output allocation failed");
     const int64_t grid = std::min<int64_t>(cdiv(m, kParseThreads), (int64_t)sm_count() * 16);
     mbr_bin_kernel<<<(unsigned)grid, kParseThreads, 0, stream>>>(
@@ -952,19 +965,19 @@ int ingest_bin(Source& src, int64_t n, float r, crt_bbox_f32* box_out, int64_t* 
 
 using namespace crt;
 
-extern "C" {
-
-int crt_read_mbr_csv_device(const char* path, int64_t n, float r, crt_bbox_f32* d_box,
-                            int64_t* n_read, crt_stream_t stream)
+// A loader call on a file; `who` names it in errors.
+static int read_mbr_file(const char* who, bool bin, const char* path, int64_t n, float r, Columns from,
+                         crt_bbox_f32* d_box, int64_t* n_read, crt_stream_t stream)
 {
-  if (!path || !d_box || n < -1) return fail(CRT_ERR_INVALID_ARG, "read_mbr_csv_device: bad arguments");
+  const std::string name(who);
+  if (!path || !d_box || n < -1) return fail(CRT_ERR_INVALID_ARG, name + ": bad arguments");
   if (n_read) *n_read = 0;
   const int fd = open(path, O_RDONLY | O_CLOEXEC);
-  if (fd < 0) return fail(CRT_ERR_INVALID_ARG, std::string("read_mbr_csv_device: cannot open ") + path);
+  if (fd < 0) return fail(CRT_ERR_INVALID_ARG, name + ": cannot open " + path);
   struct stat sb;
   if (fstat(fd, &sb) != 0 || !S_ISREG(sb.st_mode)) {
     close(fd);
-    return fail(CRT_ERR_INVALID_ARG, std::string("read_mbr_csv_device: not a regular file: ") + path);
+    return fail(CRT_ERR_INVALID_ARG, name + ": not a regular file: " + path);
   }
   int rc;
   {
@@ -972,36 +985,39 @@ int crt_read_mbr_csv_device(const char* path, int64_t n, float r, crt_bbox_f32* 
     src.fd = fd;
     src.len = (int64_t)sb.st_size;
     crt_bbox_f32 box{};
-    rc = ingest(src, n, r, true, Outputs{}, &box, n_read, (cudaStream_t)stream);
+    rc = bin ? ingest_bin(src, n, r, from, &box, n_read, (cudaStream_t)stream)
+             : ingest(src, n, r, from, Outputs{}, &box, n_read, (cudaStream_t)stream);
     if (rc == CRT_OK) *d_box = box;
   }
   close(fd);
   return rc;
 }
 
+extern "C" {
+
+int crt_read_mbr_csv_device(const char* path, int64_t n, float r, crt_bbox_f32* d_box,
+                            int64_t* n_read, crt_stream_t stream)
+{
+  return read_mbr_file("read_mbr_csv_device", false, path, n, r, Columns::kOwn, d_box, n_read, stream);
+}
+
 int crt_read_mbr_bin_device(const char* path, int64_t n, float r, crt_bbox_f32* d_box,
                             int64_t* n_read, crt_stream_t stream)
 {
-  if (!path || !d_box || n < -1) return fail(CRT_ERR_INVALID_ARG, "read_mbr_bin_device: bad arguments");
-  if (n_read) *n_read = 0;
-  const int fd = open(path, O_RDONLY | O_CLOEXEC);
-  if (fd < 0) return fail(CRT_ERR_INVALID_ARG, std::string("read_mbr_bin_device: cannot open ") + path);
-  struct stat sb;
-  if (fstat(fd, &sb) != 0 || !S_ISREG(sb.st_mode)) {
-    close(fd);
-    return fail(CRT_ERR_INVALID_ARG, std::string("read_mbr_bin_device: not a regular file: ") + path);
-  }
-  int rc;
-  {
-    Source src;
-    src.fd = fd;
-    src.len = (int64_t)sb.st_size;
-    crt_bbox_f32 box{};
-    rc = ingest_bin(src, n, r, &box, n_read, (cudaStream_t)stream);
-    if (rc == CRT_OK) *d_box = box;
-  }
-  close(fd);
-  return rc;
+  return read_mbr_file("read_mbr_bin_device", true, path, n, r, Columns::kOwn, d_box, n_read, stream);
+}
+
+// The Python loaders' forms (not part of the C interface): pool columns, freed
+// with crt_bbox_free once the caller's copies of them are complete.
+int crt_internal_read_mbr_csv_pool(const char* path, int64_t n, float r, crt_bbox_f32* d_box,
+                                   int64_t* n_read, crt_stream_t stream)
+{
+  return read_mbr_file("read_mbr_csv_device", false, path, n, r, Columns::kPool, d_box, n_read, stream);
+}
+int crt_internal_read_mbr_bin_pool(const char* path, int64_t n, float r, crt_bbox_f32* d_box,
+                                   int64_t* n_read, crt_stream_t stream)
+{
+  return read_mbr_file("read_mbr_bin_device", true, path, n, r, Columns::kPool, d_box, n_read, stream);
 }
 
 int crt_parse_mbr_csv_device(const char* text, int64_t len, int64_t n, float r, float* d_xmin,
@@ -1015,7 +1031,7 @@ int crt_parse_mbr_csv_device(const char* text, int64_t len, int64_t n, float r, 
   src.mem = len > 0 ? text : nullptr;
   src.len = len;
   Outputs out{d_xmin, d_ymin, d_xmax, d_ymax, d_id};
-  return ingest(src, n, r, false, out, nullptr, n_read, (cudaStream_t)stream);
+  return ingest(src, n, r, Columns::kCallers, out, nullptr, n_read, (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -278,8 +278,8 @@ int crt_read_mbr_csv(const char* path, int64_t n, float r, float* xmin, float* y
 /* Replaces readMBR followed by box_h2d (src/utility.cpp:5-40,
  * src/utility.cuh:42-66): the same format, values, statuses and *n_read as
  * crt_read_mbr_csv, with the records found and parsed on the GPU.  The boxes
- * land in new arrays *d_box from the device's stream-ordered pool (free with
- * crt_bbox_free or cudaFree); n = -1 reads every record of the file.  On an error nothing is allocated.
+ * land in newly cudaMalloc'd arrays *d_box (free with crt_bbox_free); n = -1
+ * reads every record of the file.  On an error nothing is allocated.
  * Records the device parser cannot convert with certainty (hex or inf/nan
  * spellings, values within a few double ulps of a float rounding boundary,
  * malformed records, ...) are parsed by the host parser, so the result is
@@ -288,7 +288,7 @@ int crt_read_mbr_csv_device(const char* path, int64_t n, float r, crt_bbox_f32* 
                             int64_t* n_read, crt_stream_t stream);
 /* Binary form of the same records (no reference counterpart: the reference
  * reads text only): a file of 28-byte little-endian records, float32 x1, y1,
- * x2, y2 then int32 id, pid, nume, read into new pool arrays *d_box
+ * x2, y2 then int32 id, pid, nume, read into newly cudaMalloc'd arrays *d_box
  * with readMBR's box [min(x1,x2) - r, max(x1,x2) + r] x [min(y1,y2) - r,
  * max(y1,y2) + r] (free with crt_bbox_free).  n = -1 reads every record; a
  * file size that is not a multiple of 28, or fewer than n records, is

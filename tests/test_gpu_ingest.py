@@ -443,3 +443,68 @@ def test_read_all_records_as_fscanf_finds_them(crt):
                 assert np.array_equal(hi[:hn], di), text
             else:
                 assert ds == _lib.CRT_ERR_INVALID_ARG and dn == hn, (text, hs, hn, ds, dn)
+
+
+def _load(path, binary):
+    L = _lib.load()
+    box = _lib.crt_bbox_f32()
+    fn = L.crt_read_mbr_bin_device if binary else L.crt_read_mbr_csv_device
+    got = ctypes.c_int64(0)
+    assert fn(str(path).encode(), -1, 0.0, ctypes.byref(box), ctypes.byref(got), None) == 0
+    return box
+
+
+@pytest.mark.parametrize("binary", [False, True], ids=["csv", "bin"])
+def test_loaded_columns_are_plain_device_allocations(crt, tmp_path, binary):
+    """crtree.h: five cudaMalloc'd arrays, so each is an allocation of its own
+    that other processes and devices can be given, in no memory pool."""
+    from curtree_b200 import datasets as D
+    b = D.uniform_boxes(5_003, seed=1)
+    path = tmp_path / "boxes"
+    path.write_bytes(D.mbr_bin_bytes(b) if binary else D.mbr_csv_text(b, seed=1))
+    box = _load(path, binary)
+    cu = ctypes.CDLL("libcuda.so.1")
+    ipc_capable, range_start, mempool = 10, 11, 17  # CU_POINTER_ATTRIBUTE_*
+
+    def attribute(which, ptr, kind):
+        v = kind(0)
+        assert cu.cuPointerGetAttribute(ctypes.byref(v), which, ctypes.c_uint64(ptr)) == 0
+        return v.value
+    for ptr in (box.xmin, box.ymin, box.xmax, box.ymax, box.id):
+        assert attribute(ipc_capable, ptr, ctypes.c_int) == 1
+        assert attribute(range_start, ptr, ctypes.c_uint64) == ptr
+        assert not attribute(mempool, ptr, ctypes.c_void_p)
+    assert _lib.load().crt_bbox_free(ctypes.byref(box)) == 0
+
+
+def test_windows_freed_behind_an_asynchronous_query(crt, tmp_path):
+    """crt_bbox_free waits for a query that still reads the loaded windows: the
+    next load may get their memory."""
+    import torch
+    from curtree_b200 import datasets as D
+    d, rt = crt.build_into(crt.BBox.from_host(D.uniform_boxes(1_000_003, seed=2)), 10)
+    paths = []
+    for k in range(2):
+        paths.append(tmp_path / f"w{k}")
+        paths[k].write_bytes(D.mbr_bin_bytes(D.uniform_windows(60_000, seed=10 + k, max_side=2e-2)))
+    want = crt.read_mbr_bin(str(paths[0]))
+    ref = crt.query(rt, d, want)
+    n = int(ref[0].numel())
+    cap = crt.query_capacity(n)
+    fid, tid = (torch.empty(cap, dtype=torch.int32, device="cuda") for _ in range(2))
+    L = _lib.load()
+    o = _lib.default_opts()
+    for _ in range(5):
+        box = _load(paths[0], True)
+        res = crt.new_result_block()
+        assert L.crt_query_into_f32(ctypes.byref(rt.s), ctypes.byref(d.c()), ctypes.byref(box), fid.data_ptr(),
+                                    tid.data_ptr(), cap, res.data_ptr(), None, ctypes.byref(o),
+                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+        assert L.crt_bbox_free(ctypes.byref(box)) == 0
+        other = _load(paths[1], True)
+        assert crt.read_result(res)["count"] == n
+        a, b = crt.PairDigest(want.sz), crt.PairDigest(want.sz)
+        a.add(fid, tid, n=n)
+        b.add(*ref)
+        assert torch.equal(a.counts, b.counts) and torch.equal(a.hashes, b.hashes)
+        assert L.crt_bbox_free(ctypes.byref(other)) == 0
