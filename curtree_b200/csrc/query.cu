@@ -186,6 +186,7 @@ constexpr int kJobs = 1 << 18;         // queue entries per launch (8 MiB)
 constexpr int kPiece = 16384;          // ids per piece
 constexpr int kShareMin = 2 * kPiece;  // ranges shorter than this stay with their finder
 constexpr size_t kJobQueueBytes = offsetof(JobQueue, entries) + sizeof(RangeJob) * kJobs;
+constexpr int kQueue = 64;  // contained runs a warp can queue (ChunkEmit)
 
 __device__ __forceinline__ void fence_sc_gpu() { asm volatile("fence.sc.gpu;" ::: "memory"); }
 
@@ -226,11 +227,13 @@ __device__ __forceinline__ int wait_piece(JobQueue* Q, const QueryCounters* ctr,
   return 0;
 }
 
-// Warp-reserved output chunks (persistent form).
+// Warp-reserved output chunks (persistent form).  kQueued: the warp queues
+// contained runs.
+template <bool kQueued>
 struct ChunkEmit {
   static constexpr bool kCountsTests = false;
   // runs of 64 boxes and more are queued (32: the same, 128: 2% slower, 256: 6%)
-  static constexpr int kSmall = 64;
+  static constexpr int kSmall = kQueued ? 64 : kSmallRange;
   int32_t* fid;
   int32_t* tid;
   long long cap;
@@ -280,18 +283,28 @@ struct ChunkEmit {
   // takes about one atomic per 1.6 ns: with one per range 10M boxes x 250k
   // windows of side 1e-2..1e-1 took 21 ms, with one per step 12.4 (and 1M
   // mixed windows 17.0 ms where runs down to 64 boxes came here, 11.2 queued).
-  int2* queue = nullptr;  // 64 entries of this warp: first slot, count
+  // Without a queue (persist_shape) a step's runs share one reservation: a kernel
+  // of its own, since a branch here cost the 16-warp shape (40 registers) 3%.
+  int2* queue = nullptr;  // kQueue entries of this warp: first slot, count
   int queued = 0;
   __device__ __forceinline__ void big_ranges(const int* bid, bool mine, long long first, long long count)
   {
     const uint32_t m = __ballot_sync(0xffffffffu, mine);
-    if (mine) queue[queued + __popc(m & lanemask_lt())] = make_int2((int)first, (int)count);
+    const int lane = (int)lane_id();
+    int2 r = make_int2((int)first, (int)count);
+    if constexpr (!kQueued) {  // this step's runs to the first lanes
+      const int at = (int)__fns(m, 0, lane + 1) & 31;
+      r = make_int2(__shfl_sync(0xffffffffu, r.x, at), __shfl_sync(0xffffffffu, r.y, at));
+      if (lane >= __popc(m)) r = make_int2(0, 0);
+      place_ranges(bid, r, __popc(m));
+      return;
+    }
+    if (mine) queue[queued + __popc(m & lanemask_lt())] = r;
     queued += __popc(m);
     __syncwarp();
     if (queued >= 32) {
       flush_ranges(bid);
       // the entries past the first 32 move down
-      const int lane = (int)lane_id();
       int2 rest = make_int2(0, 0);
       if (lane < queued) rest = queue[32 + lane];
       __syncwarp();
@@ -302,10 +315,16 @@ struct ChunkEmit {
   // Places the first 32 queued ranges (all, when there are fewer).
   __device__ __forceinline__ void flush_ranges(const int* bid)
   {
-    const int lane = (int)lane_id();
     const int n = min(queued, 32);
     if (n == 0) return;
-    const int2 r = lane < n ? queue[lane] : make_int2(0, 0);
+    place_ranges(bid, (int)lane_id() < n ? queue[lane_id()] : make_int2(0, 0), n);
+    queued -= n;
+  }
+  // Places the ranges of the first n lanes in one reservation (the other lanes'
+  // are empty).
+  __device__ __forceinline__ void place_ranges(const int* bid, int2 r, int n)
+  {
+    const int lane = (int)lane_id();
     long long x = r.y;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -319,7 +338,6 @@ struct ChunkEmit {
     for (int i = 0; i < n; i++)
       place(bid, __shfl_sync(0xffffffffu, r.x, i), __shfl_sync(0xffffffffu, r.y, i),
             (long long)nb + __shfl_sync(0xffffffffu, excl, i));
-    queued -= n;
   }
   // Copies a contained subtree's ids to its reservation at output slot nb
   // (large ones cut into pieces that idle warps copy).
@@ -566,8 +584,9 @@ __device__ __forceinline__ int split_parts_for(long long nhuge, long long warps)
 
 // kShare: range sharing (the job queue).  Its code needs registers the
 // tighter CTA shapes do not have, so only the 8-warp shape (64 registers)
-// shares ranges; the autotuner weighs the shapes against each other.
-template <int kThreads, int kMinBlocks, bool kShare>
+// shares ranges; the autotuner weighs the shapes against each other.  kQueued:
+// the warps have queues of contained runs.
+template <int kThreads, int kMinBlocks, bool kShare, bool kQueued>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
     persistent_kernel(PersistParams P)
 {
@@ -578,7 +597,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   const int warps = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
   // layout: [staged nodes: 6 arrays x stage_n x 4 B][stacks: warps x stack_cap
-  // entries][queued ranges: warps x 64]
+  // entries][queued ranges: warps x kQueue, or none]
   float* c_xmin = (float*)smem_raw;
   float* c_ymin = c_xmin + P.stage_n;
   float* c_xmax = c_ymin + P.stage_n;
@@ -630,7 +649,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 
   FrontierEntry* stack = stacks + warp * P.stack_cap;
-  int2* queue = (int2*)(stacks + warps * P.stack_cap) + warp * 64;
   int lg, lc;
   lane_map(P.T.fanout, lg, lc);
   const uint32_t* order = nullptr;
@@ -645,13 +663,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   const int split_parts = split_parts_for(nhuge, (long long)gridDim.x * warps);
   const long long nsplit = nhuge * split_parts;
   const long long ntickets = nsplit + ((P.classes ? (long long)P.ctr->nlarge : nq) - nhuge) * parts;
-  ChunkEmit emit;
+  ChunkEmit<kQueued> emit;
   emit.fid = P.fid;
   emit.tid = P.tid;
   emit.cap = P.cap;
   emit.next = &P.ctr->next;
   emit.chunk = P.chunk;
-  emit.queue = queue;
+  if constexpr (kQueued) emit.queue = (int2*)(stacks + warps * P.stack_cap) + warp * kQueue;
   emit.jobs = kShare ? P.jobs : nullptr;
   JobQueue* Q = kShare ? P.jobs : nullptr;
   // a warp counts as active from before its first ticket until it has left
@@ -688,7 +706,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     emit.begin(q);
     traverse(P.T, C, P.K, lg, lc, P.W.xmin[q], P.W.ymin[q], P.W.xmax[q], P.W.ymax[q], stack,
              P.stack_cap, emit, &P.ctr->error, part, nparts, split);
-    emit.flush_ranges(P.T.bid);
+    if constexpr (kQueued) emit.flush_ranges(P.T.bid);
   }
   if (Q) {
     __syncwarp();
@@ -1478,14 +1496,16 @@ constexpr int kDefaultChunkRoom = 4096;
 struct PersistVariant {
   int threads;
   int min_blocks;
-  bool share;  // range sharing
-  const void* fn;
+  bool share;         // range sharing
+  const void* fn[2];  // without and with queues of contained runs
 };
 
+#define CRT_VARIANT(T, B, S) \
+  {T, B, S, {(const void*)persistent_kernel<T, B, S, false>, (const void*)persistent_kernel<T, B, S, true>}}
 static const PersistVariant kVariants[] = {
-    {1024, 2, false, (const void*)persistent_kernel<1024, 2, false>},  // 64 warps/SM, 32 registers
-    {512, 3, false, (const void*)persistent_kernel<512, 3, false>},    // 48 warps/SM, 40 registers
-    {256, 4, true, (const void*)persistent_kernel<256, 4, true>},     // 32 warps/SM, 64 registers
+    CRT_VARIANT(1024, 2, false),  // 64 warps/SM, 32 registers
+    CRT_VARIANT(512, 3, false),   // 48 warps/SM, 40 registers
+    CRT_VARIANT(256, 4, true),    // 32 warps/SM, 64 registers
 };
 
 static const PersistVariant& variant_for(int warps_per_cta)
@@ -1495,36 +1515,57 @@ static const PersistVariant& variant_for(int warps_per_cta)
   return kVariants[2];  // default: 8 warps per CTA
 }
 
-static int persistent_grid(const PersistVariant& v, size_t smem)
-{
-  int per_sm = 0;
-  allow_smem(v.fn, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, v.fn, v.threads, smem);
-  if (per_sm < 1) per_sm = 1;
-  return per_sm * sm_count();
-}
-
-// Shared memory of the persistent traversal: the staged top levels (6 arrays)
-// and one frontier stack per warp.  When that does not let the variant's CTAs
-// share an SM, staging is dropped; a stack too deep for one CTA per SM is an
-// error.
+// Shared memory of the persistent traversal: the staged top levels (6 arrays),
+// one frontier stack per warp and the warps' queues of contained runs.  When
+// that does not let the variant's CTAs share an SM, staging is dropped, then the
+// CTAs per SM, and last the queues (fanout 2 in 32-warp CTAs above 2^25 boxes);
+// a stack too deep for that too is an error.  The queues go last: where they
+// cost one of an SM's CTAs (deep trees of fanout 2 to 4) batches of 50k mixed
+// windows took, with the queues and without: fanout 3, 10M boxes, 32 warps 688
+// and 711 us; fanout 2, 200k boxes, 16 warps 155 and 162; fanout 4, 30M boxes,
+// 32 warps 1090 and 1128 (100k windows of one size, side 1e-2: 1960 and 1815,
+// 274 and 285, 3620 and 3600).
 struct PersistShape {
   const PersistVariant* v;
   int stage_n;
+  bool queue;
   size_t smem;
+  const void* fn() const { return v->fn[queue]; }
 };
 
 static PersistShape persist_shape(int stack_cap, int stage_n, int warps_per_cta)
 {
   const PersistVariant& v = variant_for(warps_per_cta);
   const size_t per_sm = 227 * 1024;
-  for (int pass = 0; pass < 3; pass++) {
+  const int warps = v.threads / 32;
+  for (int pass = 0; pass < 4; pass++) {
     const int sn = pass == 0 ? stage_n : 0;
-    const size_t smem = (size_t)sn * 24 + (size_t)(v.threads / 32) * (stack_cap + 64) * sizeof(FrontierEntry);
+    const bool queue = pass < 3;
+    const size_t smem = (size_t)sn * 24 + (size_t)warps * (stack_cap * sizeof(FrontierEntry) +
+                                                           (queue ? kQueue * sizeof(int2) : 0));
     const size_t limit = pass < 2 ? per_sm / v.min_blocks - 1024 : 220 * 1024;
-    if (smem <= limit) return PersistShape{&v, sn, smem};
+    if (smem <= limit) return PersistShape{&v, sn, queue, smem};
   }
-  return PersistShape{nullptr, 0, 0};
+  return PersistShape{nullptr, 0, false, 0};
+}
+
+static int persistent_grid(const PersistShape& p)
+{
+  int per_sm = 0;
+  allow_smem(p.fn(), p.smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.fn(), p.v->threads, p.smem);
+  if (per_sm < 1) per_sm = 1;
+  return per_sm * sm_count();
+}
+
+// The shape above for tests: {shared memory (0: refused), nodes staged, whether
+// the warps have queues}.
+void persist_shape_of(int64_t nbox, int fanout, int stage_n, int warps_per_cta, int out[3])
+{
+  const PersistShape p = persist_shape(traversal_shape(nbox, fanout).stack_cap, stage_n, warps_per_cta);
+  out[0] = (int)p.smem;
+  out[1] = p.stage_n;
+  out[2] = p.queue;
 }
 
 int64_t query_capacity(int64_t pairs, const crt_query_opts& o)
@@ -1665,8 +1706,8 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
   P.jobs = S.jobs;
   L.smem = ps.smem;
   L.threads = ps.v->threads;
-  L.fn = ps.v->fn;
-  L.grid = persistent_grid(*ps.v, L.smem);
+  L.fn = ps.fn();
+  L.grid = persistent_grid(ps);
   if (P.classes) {
     L.small = P;
     // as one window's stack, with kSmallSets sets per step, a refill and the
@@ -1745,7 +1786,7 @@ static int fit_stage_nodes(const crt_rtree_f32& rt, int64_t nbox, int levels, in
 static long long max_holes_for(int stack_cap, int stage_n, int warps_per_cta)
 {
   const PersistShape ps = persist_shape(stack_cap, stage_n, warps_per_cta);
-  return (long long)persistent_grid(*ps.v, ps.smem) * (ps.v->threads / 32);
+  return (long long)persistent_grid(ps) * (ps.v->threads / 32);
 }
 
 // Warps per window of the persistent form (0 = 1); -1 for an unsupported value.

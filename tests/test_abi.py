@@ -86,3 +86,34 @@ def test_device_bytes_interface():
     from curtree_b200.rtree import _DeviceBytes
     cai = _DeviceBytes(0x1000, 64).__cuda_array_interface__
     assert cai == {"shape": (64,), "typestr": "|u1", "data": (0x1000, False), "version": 2}
+
+
+@pytest.mark.parametrize("warps,resident", [(8, 4), (16, 3), (32, 2)])
+def test_traversal_shapes_beside_the_range_queues(warps, resident):
+    """The persistent traversal's shared memory over tree depths and fanouts:
+    every tree whose stacks fit an SM by themselves is accepted, with the
+    warps' queues of contained runs wherever those fit too."""
+    L = _lib.load()
+    shape = L._ZN3crt16persist_shape_ofEliiiPi
+    shape.restype = None
+    shape.argtypes = [ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_int)]
+    seen = set()
+    for fanout in (2, 3, 4, 5, 7, 10, 16, 31, 32, 33, 48, 300, 870, 1740, 2000, 5000):
+        for n in [1, 2, 100] + [(1 << b) + d for b in range(10, 30) for d in (0, 1)]:
+            depth = max(L.crt_tree_levels(n, fanout, None, 0), 1)
+            k = max(32 // fanout, 1) if fanout <= 32 else 1
+            stacks = -(-((depth - 1) * k * fanout + 1) // 32) * 32 * 8 * warps
+            queues = 64 * 8 * warps
+            for stage in (0, 164, 2000, 4000):
+                out = (ctypes.c_int * 3)()
+                shape(n, fanout, stage, warps, out)
+                smem, staged, queue = out
+                assert (smem > 0) == (stacks <= 220 * 1024), (fanout, n)
+                if not smem:
+                    continue
+                assert smem == stacks + queues * queue + 24 * staged and staged in (0, stage)
+                assert queue == (stacks + queues <= 220 * 1024), (fanout, n)
+                one = 227 * 1024 // resident - 1024
+                assert staged == (stage if stacks + queues + 24 * stage <= one else 0)
+                seen.add((staged > 0, queue, smem <= one))
+    assert {(True, 1, True), (False, 1, True), (False, 1, False), (False, 0, False)} <= seen

@@ -161,3 +161,36 @@ def test_plain_offsets_at_scan_edges(crt, nq):
     counts = O.tree_query_stats(t, sb, q).counts
     assert np.array_equal(offs.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
     assert np.array_equal(tid.cpu().numpy(), np.repeat(np.arange(nq), counts))
+
+
+@pytest.mark.parametrize("n,fanout,warps", [((1 << 25) + 5, 2, 32), (800_003, 870, 16), (3_100_003, 1740, 8)])
+def test_stacks_that_leave_no_room_for_the_range_queues(crt, n, fanout, warps):
+    """Trees whose stacks leave the warps no room for their queues of contained
+    runs, as a query and a plan: the plain form's pairs."""
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    r = lambda n: torch.rand(n, generator=g, device="cuda") * 2 ** 15
+    nq = 2000
+
+    def boxes(n, side):
+        x, y, w = r(n), r(n), r(n) * side
+        return crt.BBox(x, y, x + w, y + w, torch.arange(n, dtype=torch.int32, device="cuda"))
+    d, rt = crt.build_into(boxes(n, 1e-4), fanout)
+    q = boxes(nq, 3e-2)
+
+    def digest(fid, tid, n=None):
+        out = crt.PairDigest(nq)
+        out.add(fid, tid, n=n)
+        return out
+    fid, tid, _ = crt.query(rt, d, q, mode=crt.CRT_QUERY_PLAIN)
+    want = digest(fid, tid)
+    got = [digest(*crt.query(rt, d, q, warps_per_cta=warps))]
+    cap = crt.query_capacity(int(fid.numel()))
+    fid, tid = (torch.empty(cap, dtype=torch.int32, device="cuda") for _ in range(2))
+    res = crt.new_result_block()
+    plan = crt.Plan(rt, d, q, fid, tid, res, warps_per_cta=warps)
+    plan.launch()
+    got.append(digest(fid, tid, crt.read_result(res)["count"]))
+    for other in got:
+        assert torch.equal(want.counts, other.counts) and torch.equal(want.hashes, other.hashes)
