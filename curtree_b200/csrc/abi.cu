@@ -75,9 +75,26 @@ static bool tree_ok(const crt_rtree_f32* t)
                          t->fanout >= 2));
 }
 
-// Pairs-per-window estimate of the last drop-in query, used to size the next
-// one's output before its exact count is known.
+// What the last drop-in query found, a hint for sizing the next one's output
+// before its exact count is known.  That query may have been another thread's,
+// on another tree, so the hint is bounded: more than kFirstSlots only up to what
+// the last query really returned.  A first size that turns out too small, or
+// that memory is too short for, costs a second run at the exact size.
 static std::atomic<double> g_pairs_per_window{64.0};
+static std::atomic<int64_t> g_last_pairs{0};
+constexpr int64_t kFirstSlots = 1 << 28;  // 1 GiB per column
+
+static int64_t first_slots(int64_t nq)
+{
+  const double most = std::max((double)kFirstSlots, 1.25 * (double)g_last_pairs.load());
+  return (int64_t)std::min(most, 1.25 * g_pairs_per_window.load() * (double)nq) + 1024;
+}
+static void remember_pairs(int64_t nq, int64_t pairs)
+{
+  if (nq <= 0) return;
+  g_pairs_per_window.store(std::max(1.0, (double)pairs / (double)nq));
+  g_last_pairs.store(pairs);
+}
 
 // The drop-in query runs into buffers from the stream-ordered pool (sized from
 // the last call's pairs per window, re-run once at the exact size if that was
@@ -97,7 +114,7 @@ static int query_dropin_dense(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_r
                               const crt_bbox_f32* d_qbox, crt_idpair* d_dq, cudaStream_t stream)
 {
   const int64_t nq = d_qbox->sz;
-  int64_t cap = (int64_t)(g_pairs_per_window.load() * (double)nq * 1.25) + 1024;
+  int64_t cap = first_slots(nq);
   int64_t pairs = 0;
   int32_t* out[2] = {nullptr, nullptr};
   auto allocate = [&](int32_t** a, int64_t slots) {
@@ -117,8 +134,13 @@ static int query_dropin_dense(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_r
     }
   };
   int rc = CRT_OK;
-  for (int attempt = 0; attempt < 2; attempt++) {
+  for (int attempt = 0; attempt < 3; attempt++) {
     rc = allocate(out, cap);
+    if (rc == CRT_ERR_OOM && attempt == 0 && cap > kSpareSlots) {
+      release(out);
+      cap = kSpareSlots;  // the run counts all pairs whatever the size
+      continue;
+    }
     if (rc == CRT_OK) rc = query_dense(*d_rt, *d_rbox, *d_qbox, out[0], out[1], cap, &pairs, stream);
     if (rc != CRT_OK || pairs <= cap) break;
     release(out);
@@ -147,7 +169,7 @@ static int query_dropin_dense(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_r
     cudaStreamSynchronize(stream);
     return rc;
   }
-  if (nq > 0) g_pairs_per_window.store(std::max(1.0, (double)pairs / (double)nq));
+  remember_pairs(nq, pairs);
   d_dq->sz = (int)pairs;
   d_dq->fid = out[0];
   d_dq->tid = out[1];
@@ -169,7 +191,7 @@ static int query_dropin(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
       return query_dropin_dense(d_rt, d_rbox, d_qbox, d_dq, stream);
     o.mode = CRT_QUERY_PLAIN;
   }
-  int64_t want = (int64_t)(g_pairs_per_window.load() * (double)nq * 1.25) + 1024;
+  int64_t want = first_slots(nq);
   crt_query_result* res = nullptr;
   if (cudaMallocAsync((void**)&res, sizeof(crt_query_result), stream) != cudaSuccess) {
     cudaGetLastError();
@@ -184,6 +206,10 @@ static int query_dropin(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
     if (cudaMallocAsync((void**)&work, 2 * sizeof(int32_t) * (size_t)cap, stream) != cudaSuccess) {
       cudaGetLastError();
       work = nullptr;
+      if (attempt == 0 && want > kSpareSlots) {
+        want = kSpareSlots;
+        continue;
+      }
       rc = fail(CRT_ERR_OOM, "query: output allocation failed");
       break;
     }
@@ -233,7 +259,7 @@ static int query_dropin(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
     cudaStreamSynchronize(stream);
     return rc;
   }
-  if (nq > 0) g_pairs_per_window.store(std::max(1.0, (double)h.count / (double)nq));
+  remember_pairs(nq, h.count);
   d_dq->sz = (int)h.count;
   d_dq->fid = fid;
   d_dq->tid = tid;
