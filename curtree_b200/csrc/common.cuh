@@ -40,20 +40,20 @@ inline int sm_count()
   return n;
 }
 
-// Lets `fn` be launched with `smem` bytes of dynamic shared memory.  The limit
-// belongs to the function, not to the launch, so callers on other threads with
-// other sizes must not lower it between this call and the launch: up to
-// kSmemAsk they all set the same one.
-constexpr size_t kSmemAsk = 200 * 1024;
-inline void allow_smem(const void* fn, size_t smem)
+// Lets `fn` be launched with dynamic shared memory.  The limit belongs to the
+// function, not to the launch, so callers on other threads with other sizes must
+// not lower it between this call and the launch: every call sets the same limit,
+// all that a CTA can have beside the kernel's static shared memory (`fixed`, an
+// upper bound of it).  A launch that asks for more is refused.
+constexpr size_t kSmemPerCta = 227 * 1024;
+inline void allow_smem(const void* fn, size_t fixed = 0)
 {
-  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)(smem > kSmemAsk ? smem : kSmemAsk));
+  cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmemPerCta - fixed));
 }
 template <typename... Args>
-inline void allow_smem(void (*fn)(Args...), size_t smem)
+inline void allow_smem(void (*fn)(Args...), size_t fixed = 0)
 {
-  allow_smem((const void*)fn, smem);
+  allow_smem((const void*)fn, fixed);
 }
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }

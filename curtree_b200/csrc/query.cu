@@ -1552,7 +1552,7 @@ static PersistShape persist_shape(int stack_cap, int stage_n, int warps_per_cta)
 static int persistent_grid(const PersistShape& p)
 {
   int per_sm = 0;
-  allow_smem(p.fn(), p.smem);
+  allow_smem(p.fn(), 1024);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, p.fn(), p.v->threads, p.smem);
   if (per_sm < 1) per_sm = 1;
   return per_sm * sm_count();
@@ -1718,7 +1718,7 @@ static TraverseLaunch make_traverse(const TreeView& T, const WindowView& W,
     L.small_warp_bytes = (int)SmallSmem::bytes(L.small.stack_cap);
     const size_t smem = (size_t)L.small_warp_bytes * kSmallWarps;
     int per_sm = 0;
-    allow_smem(small_windows_kernel, smem);
+    allow_smem(small_windows_kernel);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, small_windows_kernel, kSmallWarps * 32, smem);
     L.small_grid = std::max(per_sm, 1) * sm_count();
   }
@@ -1831,7 +1831,7 @@ int query_dense(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   const bool few = T.nlev > 1 && W.n * kDenseParts <= (int64_t)sm_count() * kPlainWarps * 4;
   const int parts = few ? kDenseParts : 1;
   const size_t smem = dense_smem(sh.stack_cap);
-  allow_smem(dense_kernel, smem);
+  allow_smem(dense_kernel);
   {
     ProfScope ps("traverse_dense", stream);
     dense_kernel<<<(unsigned)cdiv(W.n * parts, kPlainWarps), kPlainWarps * 32, smem, stream>>>(
@@ -1877,8 +1877,8 @@ static void enqueue_plain(TreeView T, const LevelTables& lt, const WindowView& W
   cudaMemsetAsync(S.head, 0, plain_zero_bytes(nq), stream);
   attach_levels(T, lt, S.head + kHeadTables, nullptr, 0, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-  allow_smem(plain_count_kernel, smem);
-  allow_smem(plain_write_kernel, smem);
+  allow_smem(plain_count_kernel);
+  allow_smem(plain_write_kernel);
   const unsigned g = (unsigned)cdiv(nq, kPlainWarps);
   if (nq > 0) {
     ProfScope ps("traverse_plain", stream);
@@ -2061,8 +2061,8 @@ int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   unsigned long long* tot = (unsigned long long*)(scr + 256);  // [3] box-by-box, [3] containment
   cudaMemsetAsync(scr, 0, 1024 + kLevelTableBytes, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
-  allow_smem(stats_kernel<false>, smem);
-  allow_smem(stats_kernel<true>, smem);
+  allow_smem(stats_kernel<false>);
+  allow_smem(stats_kernel<true>);
   if (qbox.sz > 0) {
     const unsigned g = (unsigned)cdiv(qbox.sz, kPlainWarps);
     // the reference algorithm: every leaf box under an intersecting node is tested

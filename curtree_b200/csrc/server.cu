@@ -510,7 +510,7 @@ struct Server {
     *(volatile int*)&h_ctl->shutdown = 0;
     *(volatile int*)&h_ctl->error = 0;
     std::atomic_thread_fence(std::memory_order_seq_cst);
-    cudaFuncSetAttribute(serve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem());
+    allow_smem(serve_kernel);
     serve_kernel<<<grid(), kSrvThreads, smem(), compute>>>(
         d_state, d_ctl, d_trees, d_descs, d_ctrs, d_done, slots, stack_cap,
         (unsigned long long)opts.device_wait_us * 1000ull);

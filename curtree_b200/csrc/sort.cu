@@ -323,7 +323,7 @@ void sort_passes(const SortCols& cols, int64_t n, int digits, void* zero_block, 
   // memory: started while the pass before drains, its CTAs would otherwise share
   // the first SMs that fall free
   const size_t smem = tiles <= sm_count() ? std::max<size_t>(S.smem, 116 * 1024) : S.smem;
-  allow_smem(S.fn, smem);
+  allow_smem(S.fn, 1024);
   for (int d = 0; d < digits; d++) {
     ProfScope ps("sort_pass", stream);
     uint64_t* status = (uint64_t*)(ctrl + 1) + (size_t)d * tiles * kBins;

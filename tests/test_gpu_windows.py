@@ -194,3 +194,41 @@ def test_stacks_that_leave_no_room_for_the_range_queues(crt, n, fanout, warps):
     got.append(digest(fid, tid, crt.read_result(res)["count"]))
     for other in got:
         assert torch.equal(want.counts, other.counts) and torch.equal(want.hashes, other.hashes)
+
+
+def test_plain_queries_of_two_stack_sizes_on_two_threads(crt):
+    """Two host threads query trees whose stacks take 214 KB and 7 KB of shared
+    memory: neither makes the other's launches fail."""
+    import threading
+
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(4)
+    r = lambda n: torch.rand(n, generator=g, device="cuda") * 2 ** 15
+    x, y = r(3_200_000), r(3_200_000)
+    boxes = crt.BBox(x, y, x + 5, y + 5, torch.arange(x.numel(), dtype=torch.int32, device="cuda"))
+    qx, qy = r(64), r(64)
+    q = crt.BBox(qx, qy, qx + 50, qy + 50, torch.arange(64, dtype=torch.int32, device="cuda"))
+    trees = [crt.build_into(boxes, fanout) for fanout in (1700, 16)]
+    want = [crt.query_stats(rt, d, q)["hits"] for d, rt in trees]
+    bad = []
+
+    def run(k):
+        d, rt = trees[k]
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                fid, tid = (torch.empty(1 << 18, dtype=torch.int32, device="cuda") for _ in range(2))
+                res = crt.new_result_block()
+                for _ in range(3000):
+                    crt.query_into(rt, d, q, fid, tid, res, None, crt.CRT_QUERY_PLAIN)
+                if crt.read_result(res)["count"] != want[k]:
+                    bad.append((k, "count differs"))
+        except Exception as e:  # noqa: BLE001 - reported by the main thread
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=run, args=(k,)) for k in (0, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad
