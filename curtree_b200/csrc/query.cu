@@ -916,6 +916,11 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 3)
   // batches shrink towards the end (guided self-scheduling, Polychronopoulos
   // and Kuck, 1987)
   const long long share = (long long)gridDim.x * kSmallWarps * 2;
+  // and every warp takes some eight batches: 32 neighbours on dense data can hold
+  // 300k pairs (uniform boxes, 1M windows of 10: batches of 32 720 us, of 17 626,
+  // of 4 790; 1M windows of 1200 on clustered boxes 14.9 ms with four batches a
+  // warp, 12.7 with eight)
+  const long long most = max(2ll, min((long long)kGroupWindows, nsmall / (8 * share)));
   StageEmit emit;
   emit.s_out = (int2*)(my + SmallSmem::kOut);
   emit.fid = P.fid;
@@ -924,7 +929,7 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 3)
   emit.next = &P.ctr->next;
   unsigned long long t = 0;
   while (true) {
-    const int want = (int)max(1ll, min((long long)kGroupWindows, (nsmall - (long long)t) / share));
+    const int want = (int)max(1ll, min(most, (nsmall - (long long)t) / share));
     if (lane == 0) t = atomicAdd(&P.ctr->small_ticket, (unsigned long long)want);
     t = __shfl_sync(0xffffffffu, t, 0);
     if ((long long)t >= nsmall) break;
@@ -1271,18 +1276,70 @@ __global__ void __launch_bounds__(256)
 
 // Window keys and digit histograms: the boxes' Morton key, below two class
 // bits when the windows are classed (huge, large, small; the key's two lowest
-// bits make room).  The class is by the boxes a uniform density over the
-// root's MBR gives the window: it only decides which kernel answers it.  The
-// small kernel's lead over one window per warp does not hang on its line (64,
-// 256 and 1024 boxes measured within 4% on mixed batches); the huge line
-// (windows of 4k, 8k, 16k boxes and more split) took 60k mixed windows 1.31,
-// 1.43 and 1.48 ms.  A NaN makes a window large.
-constexpr float kSmallHits = 256.f;
-constexpr float kHugeHits = 4096.f;
+// bits make room).  The class is by the boxes the window may meet, taken twice:
+// at the density of the root's MBR, and at the density where the window lies
+// (local_hits), as boxes may lie in clusters, along lines, or far from one
+// another.  It only decides which kernel answers the window, but the wrong one is
+// slow: small_windows_kernel gives a warp up to 32 neighbours, and with the
+// root's density alone, windows on dense data (10M clustered boxes, 300k windows
+// of 2600 boxes each) took 10.9 ms there, where one window per warp takes 4.8 and
+// the queries before the classes took 6.1.
+//   small  at most 256 boxes at the root's density (64, 256 and 1024 measured
+//          within 4% on mixed batches) and 128 where it lies: places denser than
+//          the rest are where the estimate is worst (256: 50k windows of
+//          7300 clustered boxes in a far larger domain 1.59 ms, 128: 1.43).
+//   huge   more than 4096 (4k, 8k, 16k boxes and more split took 60k mixed windows
+//          1.31, 1.43 and 1.48 ms); where it lies 12k (50k windows of 7300 boxes,
+//          all huge by 4k, 1.05 ms, large 1.00).
+// A window that is not ordered, or has a NaN, is never small.
+constexpr float kSmallHits = 256.f, kSmallLocal = 128.f;
+constexpr float kHugeHits = 4096.f, kHugeLocal = 3 * kHugeHits;
 
-__global__ void window_key_kernel(WindowView W, TreeView T, bool classes, QueryCounters* __restrict__ qc,
-                                  uint32_t* __restrict__ keys, SortCtrl* __restrict__ ctrl)
+// Boxes that the density where the window lies gives it: the boxes in the Morton
+// cell that holds its centre and is one to two of its sides wide (in key units),
+// times the window's share of the cell.  The count comes from the keys of
+// kSamples boxes, every n / kSamples-th one in slot order, read as a piecewise
+// linear count over the keys: the boxes are sorted, so in a dense place the
+// samples lie close together.  A set in another order gives a useless number,
+// and its windows a kernel that may not suit them.  Two searches in shared memory:
+// 1M windows 10 to 15 us of 620.
+constexpr int kSamples = 8192;
+__device__ __forceinline__ int sample_at(int i) { return i + (i >> 5); }  // apart in the banks
+
+__device__ __forceinline__ float local_hits(const uint32_t* s_key, uint32_t key, float w, float h,
+                                            float per_sample)
 {
+  const float side = fmaxf(fmaxf(w, h), 1.f);
+  const int k = min(((__float_as_int(side) + 0x7FFFFF) >> 23) - 127, 16);  // 2^k >= side
+  const float cell = (float)(1 << k);
+  const float part = fminf(1.f, w / cell) * fminf(1.f, h / cell);
+  if (k == 16) return (float)kSamples * per_sample * part;
+  const uint32_t lo = key & ~((1u << 2 * k) - 1u), hi = lo + (1u << 2 * k) - 1u;
+  int a = 0;  // samples below lo (the last one is not looked at)
+#pragma unroll
+  for (int step = kSamples / 2; step; step >>= 1)
+    if (s_key[sample_at(a + step - 1)] < lo) a += step;
+  int b = a, step = 1;  // samples up to hi
+  while (b + step < kSamples && s_key[sample_at(b + step - 1)] <= hi) {
+    b += step;
+    step <<= 1;
+  }
+  for (step >>= 1; step; step >>= 1)
+    if (b + step < kSamples && s_key[sample_at(b + step - 1)] <= hi) b += step;
+  // between the samples around each end of the cell
+  const auto within = [&](int i, uint32_t v) {  // v lies above sample i - 1, not above sample i
+    if (i == 0) return 1.f;
+    const uint32_t below = s_key[sample_at(i - 1)], span = s_key[sample_at(i)] - below;
+    return span ? fminf((float)(v - below) / (float)span, 1.f) : 1.f;
+  };
+  return fmaxf(0.f, (float)(b - a) + within(b, hi) - within(a, lo)) * per_sample * part;
+}
+
+__global__ void window_key_kernel(WindowView W, TreeView T, bool classes, const uint32_t* __restrict__ samples,
+                                  QueryCounters* __restrict__ qc, uint32_t* __restrict__ keys,
+                                  SortCtrl* __restrict__ ctrl)
+{
+  __shared__ uint32_t s_key[kSamples + kSamples / 32];
   __shared__ uint32_t sh[kDigits][kBins];
   for (int i = threadIdx.x; i < kDigits * kBins; i += blockDim.x) (&sh[0][0])[i] = 0;
   classes = classes && T.lvl_odd != nullptr && *T.lvl_odd == 0;
@@ -1291,6 +1348,16 @@ __global__ void window_key_kernel(WindowView W, TreeView T, bool classes, QueryC
     root_w = __ldg(T.nxmax) - __ldg(T.nxmin);
     root_h = __ldg(T.nymax) - __ldg(T.nymin);
   }
+  const bool local = classes && T.nbox >= kSamples;
+  if (local)
+    for (int i = 4 * threadIdx.x; i < kSamples; i += 4 * blockDim.x) {
+      const uint4 v = *reinterpret_cast<const uint4*>(samples + i);
+      uint32_t* at = s_key + sample_at(i);
+      at[0] = v.x;
+      at[1] = v.y;
+      at[2] = v.z;
+      at[3] = v.w;
+    }
   unsigned huge = 0, large = 0;  // large counts both
   __syncthreads();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < W.n;
@@ -1300,8 +1367,13 @@ __global__ void window_key_kernel(WindowView W, TreeView T, bool classes, QueryC
     bool small = false;
     if (classes) {
       const float part = fminf(1.f, (x2 - x1) / root_w) * fminf(1.f, (y2 - y1) / root_h);
-      small = part * (float)T.nbox <= kSmallHits && x2 >= x1 && y2 >= y1;
-      const bool big = T.nlev > 1 && !(part * (float)T.nbox <= kHugeHits);
+      const bool box = x2 >= x1 && y2 >= y1;
+      const float hits = part * (float)T.nbox;
+      float near = 0.f;
+      if (local && box && hits <= kHugeHits)
+        near = local_hits(s_key, k, x2 - x1, y2 - y1, (float)T.nbox / kSamples);
+      small = hits <= kSmallHits && near <= kSmallLocal && box;
+      const bool big = T.nlev > 1 && !(hits <= kHugeHits && near <= kHugeLocal);
       k = k >> 2 | (small ? 0xC0000000u : big ? 0u : 0x40000000u);
       huge += big;
     }
@@ -1371,14 +1443,14 @@ LevelTables level_tables(const crt_rtree_f32& rt, int64_t nbox)
 // is not ordinary (*odd was zeroed before; every thread that sees one stores
 // the same value).  kVec: the four arrays are 16-byte aligned; eight 16-byte
 // loads per thread are then in flight (10M boxes: 53 us with 4-byte loads, 30
-// so; the read alone takes 25).
+// so; the read alone takes 25).  Given `samples`, also the keys of kSamples boxes.
 template <bool kVec>
 __global__ void __launch_bounds__(256)
     prepare_kernel(LevelTables t, int* __restrict__ first, long long* __restrict__ span,
                    int* __restrict__ odd, const float* __restrict__ xmin,
                    const float* __restrict__ ymin, const float* __restrict__ xmax,
                    const float* __restrict__ ymax, int64_t n, QueryCounters* __restrict__ ctr,
-                   long long nq)
+                   long long nq, uint32_t* __restrict__ samples)
 {
   if (blockIdx.x == 0) {
     if (first && threadIdx.x < kMaxLevels) {
@@ -1391,6 +1463,11 @@ __global__ void __launch_bounds__(256)
   bool bad = false;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t at = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (samples && n >= kSamples)
+    for (int64_t i = at; i < kSamples; i += stride) {
+      const int64_t j = i * n / kSamples;
+      samples[i] = sort_key(xmin[j], ymin[j], xmax[j], ymax[j]);
+    }
   int64_t done = 0;
   if (kVec) {
     const auto odd4 = [](float4 a, float4 b) {
@@ -1415,14 +1492,14 @@ __global__ void __launch_bounds__(256)
 static void launch_prepare(const LevelTables& t, int* first, long long* span, int* odd,
                            const float* xmin, const float* ymin, const float* xmax,
                            const float* ymax, int64_t n, QueryCounters* ctr, int64_t nq,
-                           cudaStream_t stream)
+                           uint32_t* samples, cudaStream_t stream)
 {
   const bool vec = ((((uintptr_t)xmin) | ((uintptr_t)ymin) | ((uintptr_t)xmax) | ((uintptr_t)ymax)) & 15) == 0;
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, vec ? 2048 : 256), (int64_t)sm_count() * 8));
   if (vec)
-    prepare_kernel<true><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq);
+    prepare_kernel<true><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq, samples);
   else
-    prepare_kernel<false><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq);
+    prepare_kernel<false><<<grid, 256, 0, stream>>>(t, first, span, odd, xmin, ymin, xmax, ymax, n, ctr, nq, samples);
   CRT_LAUNCHED(1);
 }
 
@@ -1431,23 +1508,23 @@ void launch_odd_boxes(const float* xmin, const float* ymin, const float* xmax, c
 {
   cudaMemsetAsync(odd, 0, sizeof(int), stream);
   if (n > 0)
-    launch_prepare(LevelTables(), nullptr, nullptr, odd, xmin, ymin, xmax, ymax, n, nullptr, 0, stream);
+    launch_prepare(LevelTables(), nullptr, nullptr, odd, xmin, ymin, xmax, ymax, n, nullptr, 0, nullptr, stream);
 }
 
 // Puts the tables at `dev` (kLevelTableBytes, 8-byte aligned, its flag word
 // zeroed by the caller), checks the view's boxes for the shortcut, points the
 // view at both, and sets ctr->nq when ctr is given.
 static void attach_levels(TreeView& T, const LevelTables& t, void* dev, QueryCounters* ctr, int64_t nq,
-                          cudaStream_t stream)
+                          uint32_t* samples, cudaStream_t stream)
 {
   if (t.nlev == 0) {
-    if (ctr) launch_prepare(t, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, ctr, nq, stream);
+    if (ctr) launch_prepare(t, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, ctr, nq, nullptr, stream);
     return;
   }
   int* first = (int*)dev;
   long long* span = (long long*)((char*)dev + sizeof(int) * kMaxLevels);
   int* odd = (int*)((char*)dev + kLevelOddOffset);
-  launch_prepare(t, first, span, odd, T.bxmin, T.bymin, T.bxmax, T.bymax, T.nbox, ctr, nq, stream);
+  launch_prepare(t, first, span, odd, T.bxmin, T.bymin, T.bxmax, T.bymax, T.nbox, ctr, nq, samples, stream);
   T.nlev = t.nlev;
   T.lvl_first = first;
   T.lvl_span = span;
@@ -1584,6 +1661,7 @@ struct PersistScratch {
   long long* cum;
   void* sort_zero;
   SortCols cols;
+  uint32_t* samples;  // kSamples keys of the boxes
   long long max_holes;
   JobQueue* jobs;
   size_t bytes;
@@ -1594,7 +1672,7 @@ static size_t persist_scratch_bytes(int64_t max_nq, long long max_holes, bool so
   auto al = [](size_t x) { return (x + 255) / 256 * 256; };
   size_t b = kHeadBytes + 2 * al(sizeof(Hole) * max_holes) +
              al(sizeof(long long) * (max_holes + 1)) + al(kJobQueueBytes);
-  if (sort) b += al(sort_zero_bytes(max_nq)) + 4 * al(4 * (size_t)std::max<int64_t>(max_nq, 1));
+  if (sort) b += al(4 * kSamples) + al(sort_zero_bytes(max_nq)) + 4 * al(4 * (size_t)std::max<int64_t>(max_nq, 1));
   return b;
 }
 
@@ -1610,6 +1688,7 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
   S.jobs = (JobQueue*)(base + off); off += al(kJobQueueBytes);
   S.sort_zero = nullptr;
   S.cols = SortCols{};
+  S.samples = nullptr;
   if (sort) {
     S.sort_zero = base + off; off += al(sort_zero_bytes(max_nq));
     size_t kv = al(4 * (size_t)std::max<int64_t>(max_nq, 1));
@@ -1617,6 +1696,7 @@ static void persist_scratch_carve(char* base, int64_t max_nq, long long max_hole
     S.cols.key[1] = (uint32_t*)(base + off); off += kv;
     S.cols.val[0] = (uint32_t*)(base + off); off += kv;
     S.cols.val[1] = (uint32_t*)(base + off); off += kv;
+    S.samples = (uint32_t*)(base + off); off += al(4 * kSamples);
     S.cols.make_values = S.cols.drop_keys = true;
   }
   S.max_holes = max_holes;
@@ -1640,7 +1720,7 @@ static void enqueue_pre(const TreeView& T, const WindowView& W, int64_t max_nq,
   if (order) {
     const int sms = sm_count();
     int g = (int)std::min<int64_t>(cdiv(max_nq, 256), (int64_t)sms * 4);
-    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, T, classes, S.ctr, S.cols.key[0],
+    window_key_kernel<<<std::max(g, 1), 256, 0, stream>>>(W, T, classes, S.samples, S.ctr, S.cols.key[0],
                                                           sort_ctrl(S.sort_zero));
     sort_passes(S.cols, W.n, kDigits, S.sort_zero, stream);
     CRT_LAUNCHED(1);
@@ -1826,7 +1906,7 @@ int query_dense(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   }
   QueryCounters* ctr = (QueryCounters*)scr;
   cudaMemsetAsync(scr, 0, kHeadBytes, stream);
-  attach_levels(T, level_tables(rt, rbox.sz), scr + kHeadTables, nullptr, 0, stream);
+  attach_levels(T, level_tables(rt, rbox.sz), scr + kHeadTables, nullptr, 0, nullptr, stream);
   // kPlainWarps x 4 warps per SM is what the traversal's shared memory allows
   const bool few = T.nlev > 1 && W.n * kDenseParts <= (int64_t)sm_count() * kPlainWarps * 4;
   const int parts = few ? kDenseParts : 1;
@@ -1875,7 +1955,7 @@ static void enqueue_plain(TreeView T, const LevelTables& lt, const WindowView& W
   QueryCounters* ctr = (QueryCounters*)S.head;
   const int64_t nq = W.n;
   cudaMemsetAsync(S.head, 0, plain_zero_bytes(nq), stream);
-  attach_levels(T, lt, S.head + kHeadTables, nullptr, 0, stream);
+  attach_levels(T, lt, S.head + kHeadTables, nullptr, 0, nullptr, stream);
   const size_t smem = (size_t)kPlainWarps * sh.stack_cap * sizeof(FrontierEntry);
   allow_smem(plain_count_kernel);
   allow_smem(plain_write_kernel);
@@ -1954,7 +2034,7 @@ int query_into(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox
   PersistScratch S;
   persist_scratch_carve(scr, nq, max_holes, sort, S);
   cudaMemsetAsync(scr, 0, kHeadBytes, stream);
-  attach_levels(T, lt, scr + kHeadTables, S.ctr, nq, stream);
+  attach_levels(T, lt, scr + kHeadTables, S.ctr, nq, S.samples, stream);
   enqueue_pre(T, W, nq, S, sort, window_classes(T, sort), variant_for(opts.warps_per_cta).share, stream);
   cudaError_t e = launch_traverse(make_traverse(T, W, S, sort, stage_n, fid, tid, capacity, chunk,
                                                 opts.warps_per_cta, parts),
@@ -2046,6 +2126,34 @@ int query_plain_noalloc(const crt_rtree_f32& rt, const crt_bbox_f32& rbox,
   return CRT_OK;
 }
 
+// The windows' classes for tests: {huge, large, small} windows of a sorted query
+// with the library's defaults.
+int window_class_counts(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,
+                        int64_t out[3], cudaStream_t stream)
+{
+  TreeView T = make_view(rt, rbox);
+  const WindowView W{qbox.xmin, qbox.ymin, qbox.xmax, qbox.ymax, qbox.sz};
+  char* scr = nullptr;
+  if (cudaMallocAsync((void**)&scr, persist_scratch_bytes(W.n, 1, true), stream) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(CRT_ERR_OOM, "window_class_counts: scratch allocation failed");
+  }
+  PersistScratch S;
+  persist_scratch_carve(scr, W.n, 1, true, S);
+  cudaMemsetAsync(scr, 0, kHeadBytes, stream);
+  attach_levels(T, level_tables(rt, rbox.sz), scr + kHeadTables, S.ctr, W.n, S.samples, stream);
+  enqueue_pre(T, W, W.n, S, true, window_classes(T, true), false, stream);
+  QueryCounters c{};
+  cudaMemcpyAsync(&c, S.ctr, sizeof(c), cudaMemcpyDeviceToHost, stream);
+  cudaFreeAsync(scr, stream);
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  if (e != cudaSuccess) return cuda_fail(e, "window_class_counts");
+  out[0] = (int64_t)c.nhuge;
+  out[1] = (int64_t)(c.nlarge - c.nhuge);
+  out[2] = W.n - (int64_t)c.nlarge;
+  return CRT_OK;
+}
+
 int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,
                 int64_t* d_hits, int64_t* d_tested, int64_t* h_totals, cudaStream_t stream)
 {
@@ -2070,7 +2178,7 @@ int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
         T, W, sh.K, sh.stack_cap, (long long*)d_hits, (long long*)d_tested, tot, ctr);
     // this library's: contained subtrees are emitted by slot range
     TreeView Tc = T;
-    attach_levels(Tc, level_tables(rt, rbox.sz), scr + 1024, nullptr, 0, stream);
+    attach_levels(Tc, level_tables(rt, rbox.sz), scr + 1024, nullptr, 0, nullptr, stream);
     stats_kernel<true><<<g, kPlainWarps * 32, smem, stream>>>(Tc, W, sh.K, sh.stack_cap, nullptr,
                                                               nullptr, tot + 3, ctr);
     CRT_LAUNCHED(2);
@@ -2178,7 +2286,7 @@ int plan_create(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbo
   persist_scratch_carve(p->scratch, max_nq, max_holes, p->sort, p->S);
   cudaMemsetAsync(p->scratch, 0, kHeadBytes, stream);
   attach_levels(p->T, opts.no_contain ? LevelTables() : level_tables(rt, rbox.sz),
-                p->scratch + kHeadTables, p->S.ctr, max_nq, stream);
+                p->scratch + kHeadTables, p->S.ctr, max_nq, p->S.samples, stream);
   p->traverse = make_traverse(p->T, p->W, p->S, p->sort, p->stage_n, fid, tid, capacity, p->chunk,
                               opts.warps_per_cta, parts);
   // capture the whole query on a private stream; a window-sorting plan
