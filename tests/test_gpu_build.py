@@ -219,3 +219,21 @@ def test_builds_of_two_sizes_on_two_threads(crt):
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("fanout", [3, 33, 48, 64, 100, 255, 300, 592, 1000, 2048, 5000])
+def test_top_levels_of_large_fanouts(crt, fanout):
+    """Parents whose children several threads of the last CTA share (2 to 256 of
+    them), at child counts around the shares, among them NaN and signed zeros."""
+    for children in sorted({2, 3, 31, 33, 65, 127, 129, 256, 257, 500, fanout + 1, 4 * fanout + 3}):
+        if children * fanout > 3_000_000:
+            continue
+        n = (children - 1) * fanout + 1 + fanout // 3
+        b = D.uniform_boxes(n, seed=children)
+        for a, k in ((b.xmin, 5), (b.ymin, 7), (b.xmax, 11), (b.ymax, 13)):
+            a[k::97] = np.float32(0.0)
+            a[k + 1::89] = np.float32(-0.0)
+            a[3 * k::1009] = np.nan
+        d, rt, rsz = gpu_build(crt, b, fanout)
+        assert_tree_equal(crt, b, fanout, d, rt, rsz)
+        rt.free()
