@@ -1213,8 +1213,11 @@ constexpr int kMovePiece = 2048;
 __global__ void __launch_bounds__(256)
     compact_kernel(const Hole* __restrict__ h, const long long* __restrict__ cum,
                    QueryCounters* __restrict__ ctr, long long max_holes, int32_t* fid,
-                   int32_t* tid, long long cap, crt_query_result* __restrict__ res)
+                   int32_t* tid, long long cap, const SortCtrl* __restrict__ sort,
+                   crt_query_result* __restrict__ res)
 {
+  // a window order that was not finished names some windows twice
+  const int error = ctr->error ? ctr->error : sort ? sort->error : 0;
   const int nh = (int)min((long long)ctr->nholes, max_holes);
   const long long T = (long long)ctr->hits;
   const long long R = (long long)ctr->next;
@@ -1223,9 +1226,9 @@ __global__ void __launch_bounds__(256)
     res->required = T;
     res->overflow = overflow ? 1 : 0;
     res->count = overflow ? 0 : T;
-    res->error = ctr->error;
+    res->error = error;
   }
-  if (overflow || ctr->error || nh == 0) return;
+  if (overflow || error || nh == 0) return;
   // holes [0, above) start below T; B hole slots lie below T
   const int above = block_partition(nh, [&](int i) { return h[i].start < T; });
   long long B = 0;
@@ -1828,8 +1831,8 @@ static void enqueue_post(const PersistScratch& S, int32_t* fid, int32_t* tid, lo
   const int sms = sm_count();
   hole_rank_kernel<<<std::max(1, (int)cdiv(S.max_holes, kRankHoles)), kRankWarps * 32, 0, stream>>>(
       S.holes, S.sorted, S.cum, S.ctr, S.max_holes);
-  compact_kernel<<<sms * 8, 256, 0, stream>>>(S.sorted, S.cum, S.ctr, S.max_holes, fid, tid,
-                                              cap, res);
+  compact_kernel<<<sms * 8, 256, 0, stream>>>(S.sorted, S.cum, S.ctr, S.max_holes, fid, tid, cap,
+                                              S.sort_zero ? sort_ctrl(S.sort_zero) : nullptr, res);
   CRT_LAUNCHED(2);
 }
 
@@ -2152,6 +2155,29 @@ int window_class_counts(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const
   out[1] = (int64_t)(c.nlarge - c.nhuge);
   out[2] = W.n - (int64_t)c.nlarge;
   return CRT_OK;
+}
+
+// The result block of a persistent query without pairs whose traversal and window
+// order left these errors, for tests: its error, or a negative status.
+int persist_result_error(int traversal, int order, cudaStream_t stream)
+{
+  char* scr = nullptr;
+  const size_t bytes = persist_scratch_bytes(2, 1, true);
+  if (cudaMallocAsync((void**)&scr, bytes + sizeof(crt_query_result), stream) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  PersistScratch S;
+  persist_scratch_carve(scr, 2, 1, true, S);
+  crt_query_result* res = (crt_query_result*)(scr + bytes);
+  crt_query_result h{};
+  cudaMemsetAsync(scr, 0, bytes, stream);
+  cudaMemcpyAsync(&S.ctr->error, &traversal, sizeof(int), cudaMemcpyHostToDevice, stream);
+  cudaMemcpyAsync(&sort_ctrl(S.sort_zero)->error, &order, sizeof(int), cudaMemcpyHostToDevice, stream);
+  enqueue_post(S, nullptr, nullptr, 0, res, stream);
+  cudaMemcpyAsync(&h, res, sizeof(h), cudaMemcpyDeviceToHost, stream);
+  cudaFreeAsync(scr, stream);
+  return cudaStreamSynchronize(stream) == cudaSuccess ? h.error : -1;
 }
 
 int query_stats(const crt_rtree_f32& rt, const crt_bbox_f32& rbox, const crt_bbox_f32& qbox,

@@ -92,3 +92,11 @@ def test_pass_after_an_error(passes, n):
     out = passes(keys, keys, 4, error=_lib.CRT_ERR_DEVICE_TIMEOUT)
     assert np.array_equal(out[0, 0, :n].view(np.uint32), keys)
     assert (out[:, 1] == -7).all() and (out[:, :, n:] == -7).all()
+
+
+@pytest.mark.parametrize("traversal,order,want", [(0, 0, 0), (0, _lib.CRT_ERR_DEVICE_TIMEOUT, _lib.CRT_ERR_DEVICE_TIMEOUT),
+                                                  (_lib.CRT_ERR_NOT_SUPPORTED, _lib.CRT_ERR_DEVICE_TIMEOUT,
+                                                   _lib.CRT_ERR_NOT_SUPPORTED)])
+def test_error_of_a_window_order_is_reported(passes, traversal, order, want):
+    """A persistent query whose window sort gave up says so in its result."""
+    assert _lib.load()._ZN3crt20persist_result_errorEiiP11CUstream_st(traversal, order, None) == want
