@@ -91,3 +91,25 @@ def test_drop_in_batch_whose_first_size_does_not_fit(crt, nq):
         pairs.free()
         with pool_of(1 << 30):
             same_pairs(crt, rt, d, b, 16, windows(nq, side, 4))
+
+
+def test_build_whose_record_blocks_do_not_fit(crt):
+    """A set large enough for records in blocks where only the tiles' own slots
+    fit: 48 bytes a box and the sort's zeroed block, against 134 MB more."""
+    import torch
+    from cuda.bindings import runtime as rt
+    n = (1 << 23) + 4321
+    b = D.uniform_boxes(n, seed=6)
+    src, out = crt.BBox.from_host(b), None
+    with pool_of(470 << 20):
+        err, _ = rt.cudaMallocAsync(48 * n + (134 << 20), 0)
+        assert err == rt.cudaError_t.cudaErrorMemoryAllocation
+        rt.cudaGetLastError()
+        out, tree = crt.build_into(src, 10)
+        torch.cuda.synchronize()
+    sb, t = O.build(b, 10)
+    got, nodes = out.to_host(), tree.to_host()
+    assert np.array_equal(got.id, sb.id)
+    for f in ("xmin", "ymin", "xmax", "ymax"):
+        assert np.array_equal(getattr(got, f), getattr(sb, f)) and np.array_equal(getattr(nodes, f), getattr(t, f))
+    assert np.array_equal(nodes.pos, t.pos) and np.array_equal(nodes.len, t.len)

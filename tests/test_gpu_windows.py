@@ -232,3 +232,18 @@ def test_plain_queries_of_two_stack_sizes_on_two_threads(crt):
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("nq", [31, 1023, 1024, 1025, 32_767, 32_768, 32_769, 33_793])
+def test_plain_offsets_at_look_back_edges(crt, nq):
+    """Plain offsets around one tile of 1024 counts and around the 32 tiles that
+    a look-back reads at a time, with windows of no box, few and many."""
+    rng = np.random.default_rng(nq)
+    b = D.uniform_boxes(5_003, seed=3)
+    q = windows(rng, nq, (0.0, 1e-3, 2e-2))
+    d, rt = crt.build_into(crt.BBox.from_host(b), 10)
+    fid, tid, offs = crt.query(rt, d, crt.BBox.from_host(q), mode=crt.CRT_QUERY_PLAIN)
+    sb, t = O.build(b, 10)
+    counts = O.tree_query_stats(t, sb, q).counts
+    assert np.array_equal(offs.cpu().numpy(), np.concatenate([[0], np.cumsum(counts)]))
+    assert np.array_equal(tid.cpu().numpy(), np.repeat(np.arange(nq), counts))
