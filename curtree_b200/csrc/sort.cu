@@ -245,6 +245,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
       if (found)
         st_relaxed_u64(&status[(int64_t)tile * kBins + tid], kFlagIncl | (uint32_t)(excl + total));
     }
+    // The bin's pairs go to [bucket + excl, + total): out of range only where the
+    // keys are not the ones the histograms were made from (a caller's columns that
+    // change during the call).  One test per bin: one per pair took 2% of a pass.
+    if (total > 0 && (uint32_t)(bucket + excl) > (uint32_t)(n - total)) s_stop = 1;
     s_gbase[tid] = bucket + excl - binstart;
   }
   __syncthreads();
@@ -256,10 +260,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     if (full || j < tile_n) {
       const uint32_t k = s_key[j];
       const int d = s_gbase[((k ^ flip) >> shift) & 255u] + j;
-      // out of range only where the keys are not the ones the histograms were
-      // made from (a caller's columns that change during the call); the test
-      // takes 2% of a pass at 100M pairs
-      if ((uint32_t)d >= (uint32_t)n) continue;
       // evict-first: a pass's output is read once, by the next pass, and
       // the look-back status words and the next tiles' runs want L2
       if (!drop_keys) __stcs(dst_k + d, k);
