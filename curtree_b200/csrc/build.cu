@@ -339,7 +339,7 @@ __device__ __forceinline__ float4 merge_box(float4 a, float4 m)
 //
 // kFuse: the launch makes the levels above its own too.
 template <bool kLeaf, bool kFuse>
-__global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers: three CTAs per SM
+__global__ void __launch_bounds__(kLevelThreads, 3)  // 80 registers (12 bytes spilled): three CTAs per SM
     level_kernel(LevelArgs A, NodeOut N,
                  // leaf inputs/outputs
                  const uint32_t* __restrict__ vals0, const uint32_t* __restrict__ vals1,
@@ -521,10 +521,11 @@ constexpr int64_t kBlocksMin = 1 << 23;
 // Records per block: the largest power of two up to 2^16 with at least
 // kBlockShare of them in the set, so the part-filled blocks (one per top byte)
 // add at most half to the copy.  10 M boxes: 2^14 154 us of levels, 2^13 162,
-// 2^12 170; 30 M: 2^16 405, 2^15 423, 2^14 536.
+// 2^12 170; 30 M: 2^16 405, 2^15 423, 2^14 536.  A set of kBlocksMin has 2^14.
 constexpr int64_t kBlockShare = 512;
 constexpr int kBlockBitsMost = 16;
-constexpr int kBlockBitsLeast = 12;
+constexpr int kBlockBitsLeast = 14;
+static_assert(kBlocksMin >> kBlockBitsLeast >= kBlockShare, "the least suits the smallest set");
 static_assert(kEncTile <= 1 << kBlockBitsLeast, "a run crosses into at most one block");
 
 // Builds the tree of `n` boxes.  in_* may alias out_* (in-place build).

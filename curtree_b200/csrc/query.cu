@@ -764,7 +764,9 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 //      tested at once, other nodes go on through traverse_group's stack.
 // Only for packed trees over ordinary boxes: a node excluded by the bounding
 // box is excluded by each window, and (NaN aside) a child that a window meets
-// lies under nodes that it meets, so skipping those tests changes nothing.  A
+// lies under nodes that it meets, so skipping those tests changes nothing: a
+// node's MBR bounds its children's and its boxes, as in every tree a build made,
+// which the tables' test (level_tables) does not look at.  A
 // NaN in a window opens that side of the bounding box.  Hits are staged in
 // shared memory and flushed densely, one reservation per flush, so nothing is
 // left for the compaction pass.
@@ -916,10 +918,10 @@ __global__ void __launch_bounds__(kSmallWarps * 32, 3)
   // batches shrink towards the end (guided self-scheduling, Polychronopoulos
   // and Kuck, 1987)
   const long long share = (long long)gridDim.x * kSmallWarps * 2;
-  // and every warp takes some eight batches: 32 neighbours on dense data can hold
+  // and there are some sixteen batches a warp: 32 neighbours on dense data can hold
   // 300k pairs (uniform boxes, 1M windows of 10: batches of 32 720 us, of 17 626,
-  // of 4 790; 1M windows of 1200 on clustered boxes 14.9 ms with four batches a
-  // warp, 12.7 with eight)
+  // of 4 790; 1M windows of 1200 on clustered boxes 14.9 ms with eight, 12.7
+  // with sixteen)
   const long long most = max(2ll, min((long long)kGroupWindows, nsmall / (8 * share)));
   StageEmit emit;
   emit.s_out = (int2*)(my + SmallSmem::kOut);

@@ -2,11 +2,14 @@
 // bulk load (Morton keys), the window ordering and the canonical pair order.
 // The caller's key kernel fills the digit histograms and its last CTA plans
 // the passes (sort_plan, sort.cuh); every pass then is one launch that reads
-// and writes the pairs once, with decoupled look-back across tiles.
+// and writes the pairs once, with decoupled look-back across tiles (Merrill and
+// Garland, "Single-pass parallel prefix scan with decoupled look-back", 2016;
+// Adinets and Merrill, "Onesweep: a faster least significant digit radix sort
+// for GPUs", 2022, put it under a radix sort's passes).
 //
 // A pass is bound by instruction issue, the shared-memory pipe and the chain
 // ticket -> keys -> ranks -> bin scan -> look-back -> stores inside a tile, not
-// by DRAM: 100M pairs take 0.56 ms per pass, 2.9 TB/s.  What shortened the
+// by DRAM: 100M pairs take 0.57 ms per pass, 2.8 TB/s.  What shortened the
 // chain (0.67 ms before): the values go through registers, on their way while
 // the bins are scanned, instead of through a third shared-memory buffer; the
 // look-back comes after the staging, when the predecessors have mostly
@@ -282,7 +285,8 @@ struct SweepShape {
 // Tile shapes by pair count: {most pairs, shape}.  A tile's fixed cost (ticket,
 // bin scan, look-back) is a few microseconds whatever its size, so large sorts
 // want large tiles, as large as the registers hold without spills (512 threads
-// x 14; x 16 spills); small ones want enough tiles to use the SMs.  Sort of a
+// x 14; x 16 spills); small ones want enough tiles to use the SMs, and CTAs per
+// SM (256 x 8 at six: 40 registers, 28 bytes of them spilled).  Sort of a
 // build (four passes, us with event overhead), by threads x keys:
 //   pairs   256x4  256x8  256x16  384x16  512x14  512x16  512x20
 //    20k       37     43      43      49      49      52      57

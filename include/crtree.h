@@ -108,6 +108,9 @@ int crt_build_f32(crt_bbox_f32* d_box, crt_rtree_f32* d_rt, crt_stream_t stream,
  * (box id, query index) pair whose boxes intersect, in unspecified order.
  * Never overflows (the reference aborts when a 32-query block expands past
  * 1024 nodes); results past INT32_MAX pairs give CRT_ERR_OVERFLOW_INT32.
+ * The arrays may be allocated larger than the pairs (at most twice, or 64k more).
+ * Every node's MBR has to bound its children's MBRs or its boxes, as a build
+ * leaves them; boxes moved in place need a new build (see crt_query_into_f32).
  * With R_sz == 0 (a one-box tree) the box is tested directly. */
 int crt_query_f32(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
                   const crt_bbox_f32* d_qbox, crt_idpair* d_dq, crt_stream_t stream);
@@ -153,7 +156,8 @@ typedef struct {
                            beside the warps' frontier stacks are left out) */
   int warps_per_cta;    /* persistent: 8, 16 or 32 warps per CTA (0 = default) */
   int chunk;            /* persistent: output slots a warp reserves at a time (0 = default) */
-  int no_contain;       /* 1: test every box even under nodes the window contains */
+  int no_contain;       /* 1: test every box even under nodes the window contains, and every
+                           node on the way to it (see crt_query_into_f32) */
   int warps_per_window; /* persistent: warps sharing one window, each taking an equal share of
                            the root's children (1, 2 or 4; 0 = 1) */
   int reserved[1];
@@ -181,7 +185,16 @@ typedef struct {
  * (int64, nq + 1 entries, exclusive prefix) into d_offsets when non-NULL, and
  * its pairs come grouped by window in window order.  PLAIN mode with
  * d_offsets may pass d_tid = NULL: the result is then CSR (box ids of window
- * w at d_fid[d_offsets[w] .. d_offsets[w + 1])), half the bytes of pairs. */
+ * w at d_fid[d_offsets[w] .. d_offsets[w + 1])), half the bytes of pairs.
+ *
+ * Every node's MBR has to bound its children's MBRs or its boxes, as a build
+ * leaves them.  A tree of the packed node count is taken to be one: a subtree
+ * whose MBR a window contains is emitted whole, and a PERSISTENT query finds
+ * small windows' nodes for neighbouring windows together, without the test of
+ * each window against each node above.  Over a tree that does not bound its boxes
+ * (boxes moved in place, nodes made by hand) the pairs are then neither the
+ * reference's nor always the same; opts->no_contain = 1 walks such a tree node
+ * by node, as the reference does. */
 int crt_query_into_f32(const crt_rtree_f32* d_rt, const crt_bbox_f32* d_rbox,
                        const crt_bbox_f32* d_qbox, int32_t* d_fid, int32_t* d_tid,
                        int64_t capacity, crt_query_result* d_result, int64_t* d_offsets,
